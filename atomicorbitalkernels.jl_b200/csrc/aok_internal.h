@@ -69,7 +69,17 @@ struct aok_plan {
     void* d_order3 = nullptr;        // per call: the items in queue order (k_prep3c)
     int* d_segs3 = nullptr;          // per call: segment starts in d_order3 (nitems3 + 1), then the count
     int* d_key3 = nullptr;           // what d_order3/d_segs3 were built from: (n, tiles, target, counts)
-    int nitems3 = 0;
+    // contracted bases with f shells (overlap3c_moments.cu): items, order, segments and their
+    // key as above, panels and moments
+    void* d_itemsm = nullptr;
+    void* d_orderm = nullptr;
+    int* d_segsm = nullptr;
+    int* d_keym = nullptr;
+    void* d_panels3 = nullptr;
+    void* d_out3 = nullptr;          // the panels' output elements
+    void* d_mom3 = nullptr;          // moments of round3 tiles: slots3 x 32 each
+    unsigned* d_cnt3 = nullptr;      // two work counters per round
+    int nitems3 = 0, nitemsm = 0, npanels3 = 0, slots3 = 0, round3 = 0, nrounds3 = 0;
     // graph mode of the fixed-basis forward (aok_plan_set_graph): the instantiated
     // launch chain, the arguments it was captured with, a private capture stream
     bool graph_on = false;
@@ -240,3 +250,13 @@ int launch_evaluate_pb(aok_orbitals* o, void* dX, void* dzeta, void* dD, const v
                        int64_t nX, double lengthscale, cudaStream_t s);
 
 }  // namespace aok
+// overlap3c_moments*.cu: the same through moments, for contracted bases with f shells; the prep
+// picks one of the two on the device
+namespace m3 {
+int setup_moments3(aok_plan* p);
+int launch_prepm3(aok_plan* p, int64_t B, cudaStream_t side);
+int launch_moments3_f32(aok_plan* p, void* out, const void* posA, const void* posB, const void* posC, int64_t B,
+                        double lengthscale, cudaStream_t s);
+int launch_moments3_f64(aok_plan* p, void* out, const void* posA, const void* posB, const void* posC, int64_t B,
+                        double lengthscale, cudaStream_t s);
+}  // namespace m3

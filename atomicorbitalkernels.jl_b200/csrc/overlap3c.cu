@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "overlap3c_kernel.cuh"
+#include "overlap3c_prep.cuh"
 
 namespace aok {
 
@@ -91,38 +92,10 @@ __device__ __forceinline__ void prim3c_flat(FT* __restrict__ pz, FT* __restrict_
 // of one tile per unit); an item that costs more than that is a segment alone.
 // More than kOrder3Max items keep the static order, one item per segment.
 // segs: the nseg + 1 segment bounds, then nseg at [n + 1] and H at [n + 2].
-constexpr int kOrder3Max = 2048;
-constexpr int kOrder3Threads = 256;
-constexpr int kOrder3Per = kOrder3Max / kOrder3Threads;
 constexpr int kCodes3 = 27 * 8 + 1;  // (class, chunk) codes of the specialised classes, + one for the f shells
 
 __device__ __forceinline__ int code3(const Item3& it) {
     return it.cls >= kClsF3 ? kCodes3 - 1 : it.cls * 8 + it.chunk;
-}
-
-// Inclusive scan of one value per thread over the kOrder3Threads threads.
-__device__ __forceinline__ long long block_scan3(long long v, long long* wtot) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const long long t = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v += t;
-    }
-    if (lane == 31) wtot[w] = v;
-    __syncthreads();
-    if (w == 0) {
-        long long t = lane < kOrder3Threads / 32 ? wtot[lane] : 0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const long long u = __shfl_up_sync(0xffffffffu, t, o);
-            if (lane >= o) t += u;
-        }
-        if (lane < kOrder3Threads / 32) wtot[lane] = t;
-    }
-    __syncthreads();
-    if (w > 0) v += wtot[w - 1];
-    __syncthreads();
-    return v;
 }
 
 __device__ __forceinline__ void order3c_body(Item3* __restrict__ order, int* __restrict__ segs,
@@ -301,8 +274,15 @@ __global__ void __launch_bounds__(kOrder3Threads) k_prep3c(FT* __restrict__ pz, 
     pdl_wait();
 }
 
+// Contracted bases with f shells may go through moments (m3; the prep picks on the device,
+// from the counts per shell), the others go through explicit E tables.  Up to d the tables
+// win for common bases (15 functions, FP32C: 19 against 32 us for 100 elements, 117 against
+// 141 for 4,096), and with one primitive per shell (FP32C 94 against 141 us for 33 elements,
+// 184 against 226 for 400, 421 against 375 for 900).
+static bool may_moments3(const aok_plan* p) { return p->Lmax > kMaxL3Spec && p->K > 1; }
+
 int setup_overlap3c_schedule(aok_plan* p) {
-    if (p->d_items3) return AOK_OK;
+    if (p->d_key3 && (p->d_panels3 || !may_moments3(p))) return AOK_OK;
     if (p->NZ * p->NZ * p->NZ > kMaxPairs)
         return set_error(AOK_ERR_UNSUPPORTED, "3C overlap: more than 6 species (NZ^3 > 256 species triples)");
     if (p->Lmax > kMaxL3) return set_error(AOK_ERR_UNSUPPORTED, "3C overlap: shells above l = 3");
@@ -347,6 +327,7 @@ int setup_overlap3c_schedule(aok_plan* p) {
     const size_t kbytes = sizeof(int) * (size_t)(4 + ns * p->NZ);
     if ((e = cudaMalloc(&p->d_key3, kbytes)) != cudaSuccess) return cuda_status(e, "cudaMalloc(key3)");
     if ((e = cudaMemset(p->d_key3, 0xFF, kbytes)) != cudaSuccess) return cuda_status(e, "cudaMemset(key3)");
+    if (may_moments3(p)) return m3::setup_moments3(p);
     return AOK_OK;
 }
 
@@ -394,23 +375,32 @@ template <typename Bin>
 static int launch_overlap3c(aok_plan* p, void* out, const void* zeta, const void* coef, const int64_t* nprim,
                             const int64_t* prim_offset, const void* posA, const void* posB, const void* posC,
                             int64_t B, double lengthscale, cudaStream_t s, Bin bin, bool chain) {
+    const bool moments = may_moments3(p);
+    auto prep = [&](cudaStream_t on, bool pdl) {
+        const int st = launch_prep3c(p, zeta, coef, nprim, prim_offset, B, on, pdl);
+        if (st != AOK_OK || !moments) return st;
+        return m3::launch_prepm3(p, B, on);
+    };
     int st;
     if (chain) {
         // one stream: the (one-launch) binning, then the prep and the kernel, each launched
         // programmatically so that its launch overlaps its predecessor
         if ((st = bin()) != AOK_OK) return st;
-        if ((st = launch_prep3c(p, zeta, coef, nprim, prim_offset, B, s, true)) != AOK_OK) return st;
+        if ((st = prep(s, true)) != AOK_OK) return st;
     } else {
         if ((st = cuda_status(cudaEventRecord(p->ev_fork, s), "cudaEventRecord")) != AOK_OK) return st;
         if ((st = cuda_status(cudaStreamWaitEvent(p->side, p->ev_fork, 0), "cudaStreamWaitEvent")) != AOK_OK)
             return st;
-        if ((st = launch_prep3c(p, zeta, coef, nprim, prim_offset, B, p->side, false)) != AOK_OK) return st;
+        if ((st = prep(p->side, false)) != AOK_OK) return st;
         if ((st = cuda_status(cudaEventRecord(p->ev_join, p->side), "cudaEventRecord")) != AOK_OK) return st;
         if ((st = bin()) != AOK_OK) return st;
         if ((st = cuda_status(cudaStreamWaitEvent(s, p->ev_join, 0), "cudaStreamWaitEvent")) != AOK_OK) return st;
     }
-    if (p->prec == AOK_PREC_F64) return launch_ov3_f64(p, out, posA, posB, posC, lengthscale, s, chain);
-    return launch_ov3_f32(p, out, posA, posB, posC, lengthscale, s, chain);
+    st = p->prec == AOK_PREC_F64 ? launch_ov3_f64(p, out, posA, posB, posC, lengthscale, s, chain)
+                                 : launch_ov3_f32(p, out, posA, posB, posC, lengthscale, s, chain);
+    if (st != AOK_OK || !moments) return st;
+    return p->prec == AOK_PREC_F64 ? m3::launch_moments3_f64(p, out, posA, posB, posC, B, lengthscale, s)
+                                   : m3::launch_moments3_f32(p, out, posA, posB, posC, B, lengthscale, s);
 }
 
 }  // namespace aok

@@ -432,7 +432,8 @@ __device__ __forceinline__ void run_item3(const Prim3<double> pr, PTd* buf, cons
     }
 }
 
-// Classes with an f shell (la, lb or lc = 3), one routine with run-time loops:
+// Classes with an f shell (la, lb or lc = 3) of bases with few primitives (with
+// more: overlap3c_moments.cuh), one routine with run-time loops:
 // the E tables of the three axes (4 x 4 x 4 each) and the chunk's <= 100 block
 // elements live in local memory, and the recursion runs in FP64 for both
 // precisions (an FP32 record's exponent coefficients are FP64 already).  The class and chunk follow the specialised path's conventions
@@ -595,6 +596,7 @@ struct Ov3Params {
     FT scale;
     int use_scale;
     int boff[kMaxShells + 1];
+    const int* pick;     // bases with f shells: nullptr, or where the prep says that moments are taken
 };
 
 // Work unit = (segment, W tiles): a run of consecutive items of the queue order
@@ -620,6 +622,8 @@ __global__ void __launch_bounds__(kThreads3, 3) k_overlap3c(const __grid_constan
     __shared__ __align__(16) FT xbuf[(W - 1) * kSplitM3 * 32 * (sizeof(FT) == 4 ? 2 : 1)];  // split partial sums
     __shared__ unsigned claim;
     pdl_wait();  // launched programmatically after the prep: its order and the bins are complete past here
+    if constexpr (F3)
+        if (P.pick && *P.pick) return;  // through moments (overlap3c_moments.cuh)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ntiles = *P.ntiles, nseg = P.segs[P.nitems + 1], H = P.segs[P.nitems + 2];
     const unsigned ngroups = (unsigned)(ntiles + W - 1) / W;
@@ -714,6 +718,7 @@ inline int launch_ov3(aok_plan* p, void* out, const void* posA, const void* posB
     P.scale = (FT)lengthscale;
     P.use_scale = (FT)lengthscale != FT(1);
     for (int i = 0; i <= p->ns; ++i) P.boff[i] = (int)p->boff[i];
+    P.pick = p->d_panels3 ? p->d_segsm + p->nitemsm + 3 : nullptr;
     auto kern = k_overlap3c<FT, F3>;
     int occ = 0;
     const int st = kernel_prepare((const void*)kern, 0, kThreads3, &occ);
@@ -728,7 +733,7 @@ inline int launch_ov3(aok_plan* p, void* out, const void* posA, const void* posB
         kern<<<p->num_sms * std::max(occ, 1), kThreads3, 0, s>>>(P);
         e = cudaGetLastError();
     }
-    timing_end(p, s);
+    if (!P.pick) timing_end(p, s);  // else after the moment path's kernels
     return cuda_status(e, "k_overlap3c");
 }
 

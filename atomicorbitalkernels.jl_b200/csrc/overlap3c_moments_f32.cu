@@ -1,0 +1,14 @@
+// overlap3c_moments_f32.cu -- float instantiation of the 3-center kernels of bases with f
+// shells.
+#include "overlap3c_moments.cuh"
+
+namespace aok {
+namespace m3 {
+
+int launch_moments3_f32(aok_plan* p, void* out, const void* posA, const void* posB, const void* posC, int64_t B,
+                        double lengthscale, cudaStream_t s) {
+    return launch_moments3<float>(p, out, posA, posB, posC, B, lengthscale, s);
+}
+
+}  // namespace m3
+}  // namespace aok
