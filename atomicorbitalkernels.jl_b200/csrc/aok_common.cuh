@@ -11,6 +11,7 @@ namespace aok {
 constexpr int kMaxL = AOK_MAX_L;
 constexpr int kTileB = 32;          // batch elements per tile (one per lane)
 constexpr int kMaxPanels = 16;
+constexpr int kSplitItems = 24;     // 2C forward: shell pairs a panel keeps when tiles are split by panel (3 per warp)
 constexpr int kMaxShells = 64;
 constexpr int kMaxPairs = 256;     // species pairs (NZ <= 16)
 

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -207,10 +208,21 @@ int launch_overlap2c(aok_plan* p, void* out, const void* posA, const void* posB,
                      double lengthscale, cudaStream_t s);
 int launch_gb_pad(aok_plan* p, const int64_t* nprim, const int64_t* prim_offset, const void* coef,
                   const void* alpha, cudaStream_t s);
+// The forward's length in whole-tile times when the tiles of a batch of B are split into k
+// panels each over `slots` CTAs: full rounds of units, and a part for a unit's own set-up
+// (255 tiles on 296 slots: 47 us whole, 52 us in halves; 125: 40 us whole, 32 us in quarters;
+// 16 tiles on 148 slots, FP64: 55 us whole, 27 us in quarters).
+inline double split_time(int64_t B, int slots, int k) {
+    const int64_t tiles = std::max<int64_t>(1, (B + kTileB - 1) / kTileB);
+    if (tiles >= slots) return k;  // the queue balances whole tiles (512 on 296 slots: halves 6 % slower)
+    return (double)((tiles * k + slots - 1) / slots) / k + (k > 1 ? 0.2 + 0.025 * k : 0.0);
+}
 // ctas = 0, stage_req = 0: the defaults (see overlap2c.cu).
 int setup_overlap2c_schedule(aok_plan* p, int ctas = 0, size_t stage_req = 0);
-int launch_ov2_f32(aok_plan* p, void* out, const void* posA, const void* posB, double lengthscale, cudaStream_t s);
-int launch_ov2_f64(aok_plan* p, void* out, const void* posA, const void* posB, double lengthscale, cudaStream_t s);
+int launch_ov2_f32(aok_plan* p, void* out, const void* posA, const void* posB, int64_t B, double lengthscale,
+                   cudaStream_t s);
+int launch_ov2_f64(aok_plan* p, void* out, const void* posA, const void* posB, int64_t B, double lengthscale,
+                   cudaStream_t s);
 
 // compile_coef.cu
 int launch_compile_coef(aok_plan* p, void* coef, const void* zeta, const void* D, cudaStream_t s);
@@ -241,15 +253,6 @@ int launch_ov3_f32(aok_plan* p, void* out, const void* posA, const void* posB, c
                    cudaStream_t s, bool pdl);
 int launch_ov3_f64(aok_plan* p, void* out, const void* posA, const void* posB, const void* posC, double lengthscale,
                    cudaStream_t s, bool pdl);
-
-// orbitals.cu
-int launch_evaluate(aok_orbitals* o, void* P, void* dP, const void* X, const int64_t* sidx,
-                    const void* zeta, const void* D, int64_t nX, double lengthscale, cudaStream_t s);
-int launch_evaluate_pb(aok_orbitals* o, void* dX, void* dzeta, void* dD, const void* dP,
-                       const void* X, const int64_t* sidx, const void* zeta, const void* D,
-                       int64_t nX, double lengthscale, cudaStream_t s);
-
-}  // namespace aok
 // overlap3c_moments*.cu: the same through moments, for contracted bases with f shells; the prep
 // picks one of the two on the device
 namespace m3 {
@@ -260,3 +263,12 @@ int launch_moments3_f32(aok_plan* p, void* out, const void* posA, const void* po
 int launch_moments3_f64(aok_plan* p, void* out, const void* posA, const void* posB, const void* posC, int64_t B,
                         double lengthscale, cudaStream_t s);
 }  // namespace m3
+
+// orbitals.cu
+int launch_evaluate(aok_orbitals* o, void* P, void* dP, const void* X, const int64_t* sidx,
+                    const void* zeta, const void* D, int64_t nX, double lengthscale, cudaStream_t s);
+int launch_evaluate_pb(aok_orbitals* o, void* dX, void* dzeta, void* dD, const void* dP,
+                       const void* X, const int64_t* sidx, const void* zeta, const void* D,
+                       int64_t nX, double lengthscale, cudaStream_t s);
+
+}  // namespace aok

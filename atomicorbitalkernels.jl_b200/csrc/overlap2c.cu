@@ -636,6 +636,33 @@ int setup_overlap2c_schedule(aok_plan* p, int ctas, size_t stage_req) {
     }
     pcols.push_back(pcols.back() + width);
     pshell.push_back(ns);
+    // Fewer tiles than CTA slots: narrower panels, so that units of one panel of a tile
+    // (k_overlap2c, split) fill them, as long as a panel keeps kSplitItems shell pairs.
+    const int slots = p->num_sms * p->fwd_ctas;
+    int want = 1;
+    for (int k = 2; k <= ns * ns / kSplitItems; ++k)
+        if (split_time(p->max_batch, slots, k) < split_time(p->max_batch, slots, want)) want = k;
+    for (int w = std::max(1, N / std::min(want, ns)); (int)pcols.size() - 1 <= kMaxPanels && want > (int)pcols.size() - 1; ++w) {
+        std::vector<int> c{0}, sh{0};
+        width = 0;
+        for (int s = 0; s < ns; ++s) {
+            const int nb = ncart((int)p->ls[s]);
+            if (width > 0 && (width + nb > w || stride_for(width + nb) * kTileB * fsz > budget)) {
+                c.push_back(c.back() + width);
+                sh.push_back(s);
+                width = 0;
+            }
+            width += nb;
+        }
+        c.push_back(c.back() + width);
+        sh.push_back(ns);
+        if ((int)c.size() - 1 > kMaxPanels) continue;  // too narrow
+        if (c.size() > pcols.size()) {
+            pcols = c;
+            pshell = sh;
+        }
+        break;
+    }
     const int npan = (int)pcols.size() - 1;
     if (npan > kMaxPanels) return set_error(AOK_ERR_UNSUPPORTED, "basis too large for the panel schedule");
     size_t maxw = 0;
@@ -768,9 +795,8 @@ int launch_bin(aok_plan* p, const int64_t* sidxA, const int64_t* sidxB, int64_t 
 
 int launch_overlap2c(aok_plan* p, void* out, const void* posA, const void* posB, int64_t B, double lengthscale,
                      cudaStream_t s) {
-    (void)B;
-    if (p->prec == AOK_PREC_F64) return launch_ov2_f64(p, out, posA, posB, lengthscale, s);
-    return launch_ov2_f32(p, out, posA, posB, lengthscale, s);
+    if (p->prec == AOK_PREC_F64) return launch_ov2_f64(p, out, posA, posB, B, lengthscale, s);
+    return launch_ov2_f32(p, out, posA, posB, B, lengthscale, s);
 }
 
 }  // namespace aok

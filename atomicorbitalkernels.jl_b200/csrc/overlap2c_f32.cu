@@ -4,13 +4,13 @@
 
 namespace aok {
 
-int launch_ov2_f32_c3(aok_plan* p, void* out, const void* posA, const void* posB, double lengthscale,
-                      cudaStream_t s);
+int launch_ov2_f32_c3(aok_plan* p, void* out, const void* posA, const void* posB, int64_t B,
+                      double lengthscale, cudaStream_t s);
 
-int launch_ov2_f32(aok_plan* p, void* out, const void* posA, const void* posB, double lengthscale,
-                   cudaStream_t s) {
-    if (p->fwd_ctas == 3) return launch_ov2_f32_c3(p, out, posA, posB, lengthscale, s);
-    return launch_ov2<float, kThreadsF32, 2>(p, out, posA, posB, lengthscale, s);
+int launch_ov2_f32(aok_plan* p, void* out, const void* posA, const void* posB, int64_t B,
+                   double lengthscale, cudaStream_t s) {
+    if (p->fwd_ctas == 3) return launch_ov2_f32_c3(p, out, posA, posB, B, lengthscale, s);
+    return launch_ov2<float, kThreadsF32, 2>(p, out, posA, posB, B, lengthscale, s);
 }
 
 }  // namespace aok

@@ -324,8 +324,18 @@ struct Ov2Params {
     unsigned* counter;
     Panels panels;
     int N, slab_stride;
+    int split;              // panels per tile when a unit is one panel of a tile; 0: whole tiles
     unsigned stage_offset;  // byte offset of the stage in dynamic shared memory
 };
+
+// Segments [k0, k1) of panel pn of a species pair (the segments are in panel order).
+__device__ __forceinline__ int2 panel_segs(const Seg* segs, int pn) {
+    int k0 = 0;
+    while ((segs[k0].pn & (kSegPanelEnd - 1)) != pn) ++k0;
+    int k1 = k0;
+    while (segs[k1].pn < kSegPanelEnd) ++k1;
+    return make_int2(k0, k1 + 1);
+}
 
 // Copy n16 16-byte words of a packed chunk into the stage, all threads, four
 // loads in flight per thread.
@@ -366,7 +376,9 @@ __device__ __forceinline__ void tile_geo(Geo<FT>& g, int& b, const Ov2Params<FT>
 // pair whose records fit one chunk stage them once).  The next tile is
 // claimed when the last segment starts, and its geometry and first chunk are
 // fetched while the last panel streams out, so a tile starts without a wait.
-template <typename FT, int THREADS, int MINB>
+// Batches of few tiles are split further (P.split): a unit is one panel of a tile,
+// the last (widest shells) first.
+template <typename FT, int THREADS, int MINB, bool SPLIT>
 __global__ void __launch_bounds__(THREADS, MINB) k_overlap2c(const __grid_constant__ Ov2Params<FT> P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     FT* slab = reinterpret_cast<FT*>(smem_raw);
@@ -379,7 +391,13 @@ __global__ void __launch_bounds__(THREADS, MINB) k_overlap2c(const __grid_consta
     __shared__ int s_b[2][32];  // batch element of each lane, double-buffered across tiles
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int NW = THREADS / 32;
-    const int ntiles = *P.ntiles;
+    // unit u: a tile, or panel split - 1 - u / tiles of tile u % tiles
+    const int tiles = *P.ntiles, ntiles = SPLIT ? tiles * P.split : tiles;
+    auto unit_tile = [&](int u) { return SPLIT ? u % tiles : u; };
+    [[maybe_unused]] auto unit_segs = [&](int u, int pair) {
+        return panel_segs(P.segs + (size_t)pair * P.seg_stride, P.split - 1 - u / tiles);
+    };
+    [[maybe_unused]] int2 kr = make_int2(0, 0);
     int staged = -1;  // packed offset of the chunk in the stage (the same in every thread)
     // prologue: the first tile, its geometry and its first chunk
     if (threadIdx.x == 0) {
@@ -389,7 +407,8 @@ __global__ void __launch_bounds__(THREADS, MINB) k_overlap2c(const __grid_consta
     __syncthreads();
     int tile = s_tile;
     if (tile < ntiles) {
-        const int4 td = P.tiles[tile];
+        const int4 td = P.tiles[unit_tile(tile)];
+        if constexpr (SPLIT) kr = unit_segs(tile, td.x);
         if (warp == NW - 1) {
             Geo<FT> g;
             int b;
@@ -398,7 +417,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_overlap2c(const __grid_consta
             s_b[0][lane] = b;
             if (lane == 0) s_td = td;
         }
-        const Seg S0 = P.segs[(size_t)td.x * P.seg_stride];
+        const Seg S0 = P.segs[(size_t)td.x * P.seg_stride + (SPLIT ? kr.x : 0)];
         stage_chunk<THREADS>(stage, P.pk + S0.off, S0.n16);
         staged = S0.off;
     }
@@ -409,11 +428,12 @@ __global__ void __launch_bounds__(THREADS, MINB) k_overlap2c(const __grid_consta
         const int pair = td.x, cnt = td.z;
         const Geo<FT> g = s_geo[lane];
         const Seg* segs = P.segs + (size_t)pair * P.seg_stride;
-        const int nseg = P.nseg[pair];
+        const int k0 = SPLIT ? kr.x : 0, nseg = SPLIT ? kr.y : P.nseg[pair];
         FT* sl = slab + (size_t)lane * P.slab_stride;
         int next = ntiles;
-        Seg S = segs[0];
-        for (int k = 0; k < nseg; ++k) {
+        [[maybe_unused]] int2 krn = kr;
+        Seg S = segs[k0];
+        for (int k = k0; k < nseg; ++k) {
             if (k == nseg - 1 && threadIdx.x == 0) s_tile = (int)atomicAdd(P.counter, 1u);
             for (;;) {
                 int it = 0;
@@ -429,7 +449,8 @@ __global__ void __launch_bounds__(THREADS, MINB) k_overlap2c(const __grid_consta
             if (k == nseg - 1) {
                 next = s_tile;
                 if (next < ntiles) {
-                    tdn = P.tiles[next];
+                    tdn = P.tiles[unit_tile(next)];
+                    if constexpr (SPLIT) krn = unit_segs(next, tdn.x);
                     if (warp == NW - 1) {  // the next tile's geometry, ahead of this warp's share of the stores
                         Geo<FT> gn;
                         int bn;
@@ -465,7 +486,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_overlap2c(const __grid_consta
                     staged = Sn.off;
                 }
             } else if (next < ntiles) {
-                const Seg S0 = P.segs[(size_t)tdn.x * P.seg_stride];
+                const Seg S0 = P.segs[(size_t)tdn.x * P.seg_stride + (SPLIT ? krn.x : 0)];
                 if (S0.off != staged) {
                     stage_chunk<THREADS>(stage, P.pk + S0.off, S0.n16);
                     staged = S0.off;
@@ -476,12 +497,13 @@ __global__ void __launch_bounds__(THREADS, MINB) k_overlap2c(const __grid_consta
             S = Sn;
         }
         tile = next;
+        if constexpr (SPLIT) kr = krn;
         buf ^= 1;
     }
 }
 
 template <typename FT, int THREADS, int MINB>
-inline int launch_ov2(aok_plan* p, void* out, const void* posA, const void* posB, double lengthscale,
+inline int launch_ov2(aok_plan* p, void* out, const void* posA, const void* posB, int64_t B, double lengthscale,
                       cudaStream_t s) {
     Ov2Params<FT> P;
     memset(&P, 0, sizeof(P));
@@ -501,10 +523,12 @@ inline int launch_ov2(aok_plan* p, void* out, const void* posA, const void* posB
     P.panels = p->panels;
     P.N = (int)p->N;
     P.slab_stride = (int)p->slab_stride;
+    const int slots = p->num_sms * MINB;
+    P.split = split_time(B, slots, p->panels.n) < split_time(B, slots, 1) ? p->panels.n : 0;
     const size_t slab = (p->smem_bytes + 15) / 16 * 16;
     P.stage_offset = (unsigned)slab;
     const size_t smem = slab + p->stage_bytes;
-    auto kern = k_overlap2c<FT, THREADS, MINB>;
+    auto kern = P.split ? k_overlap2c<FT, THREADS, MINB, true> : k_overlap2c<FT, THREADS, MINB, false>;
     const int st = kernel_prepare((const void*)kern, smem, THREADS, nullptr);
     if (st != AOK_OK) return st;
     timing_begin(p, s);
