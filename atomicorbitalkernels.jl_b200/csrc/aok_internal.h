@@ -185,11 +185,14 @@ struct BinBufs {
     void* zero3 = nullptr;
     void* zero3b = nullptr;
     int zero3_bytes = 0;
+    // the second launch programmatically after the first: where the binning is alone on the
+    // device (beside record preparations on the side stream it loses more than the launch)
+    bool pdl = false;
 };
 constexpr int kBinMaxBlocksHost = 512;
 int launch_bin_into(const BinBufs& bb, const int64_t* sidxA, const int64_t* sidxB, int64_t B, int NZ,
                     cudaStream_t s);
-int launch_bin(aok_plan* p, const int64_t* sidxA, const int64_t* sidxB, int64_t B, cudaStream_t s);
+int launch_bin(aok_plan* p, const int64_t* sidxA, const int64_t* sidxB, int64_t B, cudaStream_t s, bool pdl = false);
 // Binning by species triple (sidxC given): keys ((a-1) NZ + (b-1)) NZ + (c-1), NZ^3 <= 256.
 int launch_bin3_into(const BinBufs& bb, const int64_t* sidxA, const int64_t* sidxB, const int64_t* sidxC,
                      int64_t B, int NZ, cudaStream_t s);
@@ -204,8 +207,10 @@ int launch_overlap2c_dpos(aok_plan* p, void* dA, void* dB, const void* dS, const
                           const int64_t* sidxA, const int64_t* sidxB, const void* posA, const void* posB, int64_t B,
                           double lengthscale, cudaStream_t s);
 int launch_prep_pb(aok_plan* p, const void* zeta, const void* coef, int keep_absent, cudaStream_t s);
+// pdl: launched with programmatic serialisation after the binning (or the record packing) on
+// the same stream
 int launch_overlap2c(aok_plan* p, void* out, const void* posA, const void* posB, int64_t B,
-                     double lengthscale, cudaStream_t s);
+                     double lengthscale, cudaStream_t s, bool pdl = false);
 int launch_gb_pad(aok_plan* p, const int64_t* nprim, const int64_t* prim_offset, const void* coef,
                   const void* alpha, cudaStream_t s);
 // The forward's length in whole-tile times when the tiles of a batch of B are split into k
@@ -220,9 +225,9 @@ inline double split_time(int64_t B, int slots, int k) {
 // ctas = 0, stage_req = 0: the defaults (see overlap2c.cu).
 int setup_overlap2c_schedule(aok_plan* p, int ctas = 0, size_t stage_req = 0);
 int launch_ov2_f32(aok_plan* p, void* out, const void* posA, const void* posB, int64_t B, double lengthscale,
-                   cudaStream_t s);
+                   cudaStream_t s, bool pdl);
 int launch_ov2_f64(aok_plan* p, void* out, const void* posA, const void* posB, int64_t B, double lengthscale,
-                   cudaStream_t s);
+                   cudaStream_t s, bool pdl);
 
 // compile_coef.cu
 int launch_compile_coef(aok_plan* p, void* coef, const void* zeta, const void* D, cudaStream_t s);

@@ -263,8 +263,8 @@ static int overlap2c_graph(aok_plan* p, void* out, const void* posA, const void*
     if (!same) {
         if (!p->cap) AOK_TRY(cuda_status(cudaStreamCreateWithFlags(&p->cap, cudaStreamNonBlocking), "cudaStreamCreate"));
         AOK_TRY(cuda_status(cudaStreamBeginCapture(p->cap, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture"));
-        int st = launch_bin(p, sidxA, sidxB, B, p->cap);
-        if (st == AOK_OK) st = launch_overlap2c(p, out, posA, posB, B, lengthscale, p->cap);
+        int st = launch_bin(p, sidxA, sidxB, B, p->cap, true);
+        if (st == AOK_OK) st = launch_overlap2c(p, out, posA, posB, B, lengthscale, p->cap, true);
         cudaGraph_t g = nullptr;
         const cudaError_t e = cudaStreamEndCapture(p->cap, &g);
         if (st != AOK_OK || e != cudaSuccess) {
@@ -312,7 +312,8 @@ int aok_overlap2c(aok_plan* p, void* out, const void* zeta, const void* coef, co
     } else {
         if (!p->basis_set) return set_error(AOK_ERR_INVALID, "aok_overlap2c: no zeta/coef and no aok_plan_set_basis");
         if (p->graph_on && p->ev.empty()) return overlap2c_graph(p, out, posA, posB, sidxA, sidxB, B, lengthscale, s);
-        AOK_TRY(launch_bin(p, sidxA, sidxB, B, s));
+        AOK_TRY(launch_bin(p, sidxA, sidxB, B, s, true));
+        return launch_overlap2c(p, out, posA, posB, B, lengthscale, s, true);
     }
     return launch_overlap2c(p, out, posA, posB, B, lengthscale, s);
 }
@@ -453,10 +454,12 @@ int aok_overlap2c_gb(aok_plan* p, void* out, const int64_t* nprim, const int64_t
         return set_error(AOK_ERR_INVALID, "aok_overlap2c_gb: null pointer");
     cudaStream_t s = (cudaStream_t)stream;
     p->basis_set = false;
-    AOK_TRY(launch_gb_pad(p, nprim, prim_offset, coef, alpha, s));
-    AOK_TRY(launch_prep2c(p, p->d_gb_zeta, p->d_gb_coef, s));
+    // one stream: bins, padding, records and the kernel, each launched programmatically after
+    // its predecessor
     AOK_TRY(launch_bin(p, nullptr, nullptr, B, s));
-    return launch_overlap2c(p, out, posA, posB, B, 1.0, s);
+    AOK_TRY(launch_gb_pad(p, nprim, prim_offset, coef, alpha, s));
+    AOK_TRY(launch_prep2c(p, p->d_gb_zeta, p->d_gb_coef, s, true));
+    return launch_overlap2c(p, out, posA, posB, B, 1.0, s, true);
 }
 
 static int overlap2c_pullback(aok_plan* p, void* out0, void* out1, const void* dS, const void* zeta,

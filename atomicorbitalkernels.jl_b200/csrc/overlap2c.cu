@@ -57,18 +57,21 @@ template <typename FT>
 __global__ void k_gb_pad(FT* __restrict__ zeta, FT* __restrict__ coef, const int64_t* __restrict__ nprim,
                          const int64_t* __restrict__ off, const FT* __restrict__ c, const FT* __restrict__ a,
                          int ns, int K, int* err) {
+    pdl_trigger();  // the record packing may launch now (it waits for this grid's end)
     int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= ns * K) return;
-    int s = q % ns, k = q / ns;
-    int64_t n = nprim[s];
-    if (n > K || n < 0) atomicCAS(err, 0, AOK_ERR_INVALID);
-    if (k < n && k < K) {
-        zeta[q] = a[off[s] + k];
-        coef[q] = c[off[s] + k];
-    } else {
-        zeta[q] = FT(1);
-        coef[q] = FT(0);
+    if (q < ns * K) {
+        int s = q % ns, k = q / ns;
+        int64_t n = nprim[s];
+        if (n > K || n < 0) atomicCAS(err, 0, AOK_ERR_INVALID);
+        if (k < n && k < K) {
+            zeta[q] = a[off[s] + k];
+            coef[q] = c[off[s] + k];
+        } else {
+            zeta[q] = FT(1);
+            coef[q] = FT(0);
+        }
     }
+    pdl_wait();  // launched after the bins: they are complete once this grid is
 }
 
 // --------------------------------------------------------------------------
@@ -176,7 +179,8 @@ __global__ void __launch_bounds__(256) k_pack2c(float4* __restrict__ pk, Seg* __
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int NW = 8;
     const int npan = panels.n;
-    pdl_wait();  // coef may come from the k_compile_coef launched just before
+    pdl_trigger();  // a programmatic successor may launch now (it waits for this grid's end)
+    pdl_wait();  // coef may come from the k_compile_coef or k_gb_pad launched just before
     if (tid <= npan) {
         s_item0[tid] = panels.item0[tid];
         s_col0[tid] = panels.col0[tid];
@@ -421,6 +425,7 @@ __global__ void __launch_bounds__(kBinThreads) k_bin_count(const int64_t* __rest
                                                             int* __restrict__ err, void* zero3, void* zero3b,
                                                             int zero3_bytes) {
     __shared__ int hist[kMaxPairs];
+    pdl_trigger();  // the scatter may launch now (it waits for this grid's end)
     for (int k = threadIdx.x; k < np; k += blockDim.x) hist[k] = 0;
     __syncthreads();
     const int c0 = blockIdx.x * chunk, c1 = min(B, c0 + chunk);
@@ -438,6 +443,7 @@ __global__ void __launch_bounds__(kBinThreads) k_bin_count(const int64_t* __rest
 }
 
 constexpr int kBinWarps = kBinThreads / 32;
+constexpr int kBinKeys = 2;  // a chunk of 512 elements: 64 per warp
 __global__ void __launch_bounds__(kBinThreads) k_bin_scatter(const int64_t* __restrict__ sidxA,
                                                               const int64_t* __restrict__ sidxB,
                                                               const int64_t* __restrict__ sidxC, int B, int NZ,
@@ -449,6 +455,29 @@ __global__ void __launch_bounds__(kBinThreads) k_bin_scatter(const int64_t* __re
     __shared__ int before[kMaxPairs], tot[kMaxPairs], base[kMaxPairs], tbase[kMaxPairs + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nblk = gridDim.x, me = blockIdx.x;
+    // stable scatter of this block's chunk: warp w owns a contiguous sub-range.  Its keys and
+    // their counts need nothing of the first launch, so they come before the wait; up to
+    // kBinKeys rounds of keys stay in registers.
+    const int sub = (chunk + kBinWarps - 1) / kBinWarps;
+    const int c0 = me * chunk + warp * sub;
+    const int c1 = min(min(B, (me + 1) * chunk), c0 + sub);
+    for (int k = lane; k < np; k += 32) wcount[warp][k] = 0;
+    __syncwarp();
+    auto count = [&](int key) {
+        const unsigned peers = __match_any_sync(0xffffffffu, key);
+        if (key >= 0 && lane == __ffs(peers) - 1) wcount[warp][key] += __popc(peers);
+        __syncwarp();
+    };
+    int keys[kBinKeys];
+#pragma unroll
+    for (int i = 0; i < kBinKeys; ++i) keys[i] = pair_key(sidxA, sidxB, sidxC, c0 + 32 * i + lane, c1, NZ, err);
+#pragma unroll
+    for (int i = 0; i < kBinKeys; ++i)
+        if (c0 + 32 * i < c1) count(keys[i]);
+    for (int b0 = c0 + 32 * kBinKeys; b0 < c1; b0 += 32) count(pair_key(sidxA, sidxB, sidxC, b0 + lane, c1, NZ, err));
+    // launched programmatically after the counts; no early trigger: the overlap kernel's CTAs want
+    // another split of shared memory and L1, and this kernel's tail grew from 5 to 9 us beside them
+    pdl_wait();
     // per key: elements in earlier blocks, and the total (integer sums, so the
     // order of the shared atomics does not matter)
     for (int k = threadIdx.x; k < np; k += blockDim.x) {
@@ -481,18 +510,33 @@ __global__ void __launch_bounds__(kBinThreads) k_bin_scatter(const int64_t* __re
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (warp == 0) {
+        // first element and first tile of every key, 32 keys at a time
         int acc = 0, tacc = 0;
-        for (int q = 0; q < np; ++q) {
-            base[q] = acc;
-            tbase[q] = tacc;
-            acc += tot[q];
-            tacc += (tot[q] + kTileB - 1) / kTileB;
+        for (int q0 = 0; q0 < np; q0 += 32) {
+            const int q = q0 + lane, v = q < np ? tot[q] : 0, tv = (v + kTileB - 1) / kTileB;
+            int i = v, ti = tv;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int x = __shfl_up_sync(0xffffffffu, i, o), y = __shfl_up_sync(0xffffffffu, ti, o);
+                if (lane >= o) {
+                    i += x;
+                    ti += y;
+                }
+            }
+            if (q < np) {
+                base[q] = acc + i - v;
+                tbase[q] = tacc + ti - tv;
+            }
+            acc += __shfl_sync(0xffffffffu, i, 31);
+            tacc += __shfl_sync(0xffffffffu, ti, 31);
         }
-        tbase[np] = tacc;
-        if (me == 0) {
-            *ntiles = tacc;
-            *counter = 0u;
+        if (lane == 0) {
+            tbase[np] = tacc;
+            if (me == 0) {
+                *ntiles = tacc;
+                *counter = 0u;
+            }
         }
     }
     __syncthreads();
@@ -505,18 +549,6 @@ __global__ void __launch_bounds__(kBinThreads) k_bin_scatter(const int64_t* __re
         const int off = (t - tbase[k]) * kTileB;
         tiles[t] = make_int4(k, base[k] + off, min(kTileB, tot[k] - off), 0);
     }
-    // stable scatter of this block's chunk: warp w owns a contiguous sub-range
-    const int sub = (chunk + kBinWarps - 1) / kBinWarps;
-    const int c0 = me * chunk + warp * sub;
-    const int c1 = min(min(B, (me + 1) * chunk), c0 + sub);
-    for (int k = lane; k < np; k += 32) wcount[warp][k] = 0;
-    __syncwarp();
-    for (int b0 = c0; b0 < c1; b0 += 32) {
-        const int key = pair_key(sidxA, sidxB, sidxC, b0 + lane, c1, NZ, err);
-        const unsigned peers = __match_any_sync(0xffffffffu, key);
-        if (key >= 0 && lane == __ffs(peers) - 1) wcount[warp][key] += __popc(peers);
-        __syncwarp();
-    }
     __syncthreads();
     for (int k = threadIdx.x; k < np; k += blockDim.x) {
         int acc = base[k] + before[k];
@@ -527,15 +559,18 @@ __global__ void __launch_bounds__(kBinThreads) k_bin_scatter(const int64_t* __re
         }
     }
     __syncthreads();
-    for (int b0 = c0; b0 < c1; b0 += 32) {
-        const int b = b0 + lane;
-        const int key = pair_key(sidxA, sidxB, sidxC, b, c1, NZ, err);
+    auto put = [&](int b, int key) {
         const unsigned peers = __match_any_sync(0xffffffffu, key);
         if (key >= 0) perm[wcount[warp][key] + __popc(peers & ((1u << lane) - 1u))] = b;
         __syncwarp();
         if (key >= 0 && lane == __ffs(peers) - 1) wcount[warp][key] += __popc(peers);
         __syncwarp();
-    }
+    };
+#pragma unroll
+    for (int i = 0; i < kBinKeys; ++i)
+        if (c0 + 32 * i < c1) put(c0 + 32 * i + lane, keys[i]);
+    for (int b0 = c0 + 32 * kBinKeys; b0 < c1; b0 += 32)
+        put(b0 + lane, pair_key(sidxA, sidxB, sidxC, b0 + lane, c1, NZ, err));
 }
 
 // Single species (or no indices): every element in key 0, in batch order.  The
@@ -726,15 +761,15 @@ int launch_gb_pad(aok_plan* p, const int64_t* nprim, const int64_t* prim_offset,
                   const void* alpha, cudaStream_t s) {
     int n = (int)(p->ns * p->K);
     int th = 128, bl = (n + th - 1) / th;
-    if (p->prec == AOK_PREC_F64)
-        k_gb_pad<double><<<bl, th, 0, s>>>((double*)p->d_gb_zeta, (double*)p->d_gb_coef, nprim, prim_offset,
-                                           (const double*)coef, (const double*)alpha, (int)p->ns, (int)p->K,
-                                           p->d_err);
-    else
-        k_gb_pad<float><<<bl, th, 0, s>>>((float*)p->d_gb_zeta, (float*)p->d_gb_coef, nprim, prim_offset,
-                                          (const float*)coef, (const float*)alpha, (int)p->ns, (int)p->K,
-                                          p->d_err);
-    return cuda_status(cudaGetLastError(), "k_gb_pad");
+    auto go = [&](auto kern, auto z, auto c, auto pc, auto pa) {
+        return launch_pdl(kern, dim3(bl), dim3(th), 0, s, z, c, nprim, prim_offset, pc, pa, (int)p->ns, (int)p->K,
+                          p->d_err);
+    };
+    const cudaError_t e =
+        p->prec == AOK_PREC_F64
+            ? go(k_gb_pad<double>, (double*)p->d_gb_zeta, (double*)p->d_gb_coef, (const double*)coef, (const double*)alpha)
+            : go(k_gb_pad<float>, (float*)p->d_gb_zeta, (float*)p->d_gb_coef, (const float*)coef, (const float*)alpha);
+    return cuda_status(e, "k_gb_pad");
 }
 
 int launch_prep2c(aok_plan* p, const void* zeta, const void* coef, cudaStream_t s, bool pdl) {
@@ -777,6 +812,11 @@ int launch_bin3_into(const BinBufs& bb, const int64_t* sidxA, const int64_t* sid
     k_bin_count<<<nblk, kBinThreads, 0, s>>>(sidxA, sidxB, sidxC, (int)B, NZ, np, chunk, bb.blockhist, bb.err,
                                              bb.zero3, bb.zero3b, bb.zero3_bytes);
     AOK_TRY_ST(cuda_status(cudaGetLastError(), "k_bin_count"));
+    if (bb.pdl)
+        return cuda_status(launch_pdl(k_bin_scatter, dim3(nblk), dim3(kBinThreads), 0, s, sidxA, sidxB, sidxC, (int)B, NZ,
+                                      np, chunk, (const int*)bb.blockhist, bb.perm, bb.tiles, bb.ntiles, bb.tbase,
+                                      bb.counter, bb.err),
+                           "k_bin_scatter");
     k_bin_scatter<<<nblk, kBinThreads, 0, s>>>(sidxA, sidxB, sidxC, (int)B, NZ, np, chunk, bb.blockhist, bb.perm,
                                                bb.tiles, bb.ntiles, bb.tbase, bb.counter, bb.err);
     return cuda_status(cudaGetLastError(), "k_bin_scatter");
@@ -787,16 +827,17 @@ int launch_bin_into(const BinBufs& bb, const int64_t* sidxA, const int64_t* sidx
     return launch_bin3_into(bb, sidxA, sidxB, nullptr, B, NZ, s);
 }
 
-int launch_bin(aok_plan* p, const int64_t* sidxA, const int64_t* sidxB, int64_t B, cudaStream_t s) {
+int launch_bin(aok_plan* p, const int64_t* sidxA, const int64_t* sidxB, int64_t B, cudaStream_t s, bool pdl) {
     ++p->gen;  // the plan's bins change
-    const BinBufs bb{p->d_perm, p->d_tiles, p->d_ntiles, p->d_tbase, p->d_counter, p->d_blockhist, p->d_err};
+    BinBufs bb{p->d_perm, p->d_tiles, p->d_ntiles, p->d_tbase, p->d_counter, p->d_blockhist, p->d_err};
+    bb.pdl = pdl;
     return launch_bin_into(bb, sidxA, sidxB, B, (int)p->NZ, s);
 }
 
 int launch_overlap2c(aok_plan* p, void* out, const void* posA, const void* posB, int64_t B, double lengthscale,
-                     cudaStream_t s) {
-    if (p->prec == AOK_PREC_F64) return launch_ov2_f64(p, out, posA, posB, B, lengthscale, s);
-    return launch_ov2_f32(p, out, posA, posB, B, lengthscale, s);
+                     cudaStream_t s, bool pdl) {
+    if (p->prec == AOK_PREC_F64) return launch_ov2_f64(p, out, posA, posB, B, lengthscale, s, pdl);
+    return launch_ov2_f32(p, out, posA, posB, B, lengthscale, s, pdl);
 }
 
 }  // namespace aok

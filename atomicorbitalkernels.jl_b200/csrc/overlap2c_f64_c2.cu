@@ -5,8 +5,8 @@
 namespace aok {
 
 int launch_ov2_f64_c2(aok_plan* p, void* out, const void* posA, const void* posB, int64_t B,
-                      double lengthscale, cudaStream_t s) {
-    return launch_ov2<double, kThreadsF64, 2>(p, out, posA, posB, B, lengthscale, s);
+                      double lengthscale, cudaStream_t s, bool pdl) {
+    return launch_ov2<double, kThreadsF64, 2>(p, out, posA, posB, B, lengthscale, s, pdl);
 }
 
 }  // namespace aok
