@@ -19,10 +19,10 @@
 // writes.
 //
 // Scheduling: the batch is binned by species pair (tiles of 32 elements of one
-// pair, as the forward); a CTA of 8 warps takes a tile, lane = batch element.
+// pair, as the forward); a CTA of W warps takes a tile, lane = batch element.
 // The warps take the pair's shell pairs round-robin from a list ordered
 // heaviest class first; each lane accumulates its element's dAB over its
-// warp's shell pairs, and the 8 warp partials are added in warp order, so the
+// warp's shell pairs, and the W warp partials are added in warp order, so the
 // result does not depend on scheduling.  Records (FP64-computed, per
 // (species pair, shell pair), only pairs with both coefficients non-zero):
 // mu and w rb^al ra^be q^ga per used moment slot.
@@ -135,18 +135,38 @@ struct DposParams {
     int boff[kMaxShells + 1];
 };
 
-constexpr int kDposWarps = 8;
+// FP32: two CTAs of 8 warps per SM (<= 128 registers); FP64: one of 16 (4,000 pairs of 33
+// functions: 164 -> 121 us, of one of 8).  Bound by the latency of records and cotangent
+// rows: reading the records by 16-byte words took 8,191 pairs FP32 from 71 to 70 us, and
+// staging the cotangent panels through shared memory by cp.async lost (91 us).
+template <typename FT> constexpr int kDposWarps = sizeof(FT) == 4 ? 8 : 16;
 
-// exp(-mu R^2) of a record, and mu
-__device__ __forceinline__ float dp_exp(const DPf* r, float R2, float R2lo, float& mu) {
+// exp(-mu R^2) of a record, mu, and its slot values by whole 16-byte words.
+template <int NV>
+__device__ __forceinline__ float dp_read(const DPf* r, float R2, float R2lo, float& mu, float (&v)[8]) {
     const float4 h = __ldg(reinterpret_cast<const float4*>(r));
+#pragma unroll
+    for (int w = 0; w < (NV + 3) / 4; ++w) {
+        const float4 q = __ldg(reinterpret_cast<const float4*>(r) + 1 + w);
+        v[4 * w] = q.x;
+        v[4 * w + 1] = q.y;
+        v[4 * w + 2] = q.z;
+        v[4 * w + 3] = q.w;
+    }
     mu = h.z;
     const float xh = h.x * R2;
     const float xl = fmaf(h.x, R2, -xh) + fmaf(h.y, R2, h.x * R2lo);
     return ex2_approx(-xh) * fmaf(-0.6931471805599453f, xl, 1.f);
 }
-__device__ __forceinline__ double dp_exp(const DPd* r, double R2, double, double& mu) {
+template <int NV>
+__device__ __forceinline__ double dp_read(const DPd* r, double R2, double, double& mu, double (&v)[8]) {
     mu = __ldg(&r->mu);
+#pragma unroll
+    for (int w = 0; w < (NV + 1) / 2; ++w) {
+        const double2 q = __ldg(reinterpret_cast<const double2*>(r) + 1 + w);
+        v[2 * w] = q.x;
+        v[2 * w + 1] = q.y;
+    }
     return exp(-mu * R2);
 }
 
@@ -162,14 +182,13 @@ __device__ __noinline__ void dpos_item(const typename DPT<FT>::type* __restrict_
 #pragma unroll
     for (int j = 0; j < NV; ++j) Mv[j] = Nv[j] = FT(0);
     for (int r = 0; r < nrec; ++r) {
-        FT mu;
-        const FT e = dp_exp(rec + r, geo.R2, R2lo, mu);
+        FT mu, v[8];
+        const FT e = dp_read<NV>(rec + r, geo.R2, R2lo, mu, v);
         const FT em = e * mu;
 #pragma unroll
         for (int j = 0; j < NV; ++j) {
-            const FT v = __ldg(&rec[r].v[j]);
-            Mv[j] = fma(e, v, Mv[j]);
-            Nv[j] = fma(em, v, Nv[j]);
+            Mv[j] = fma(e, v[j], Mv[j]);
+            Nv[j] = fma(em, v[j], Nv[j]);
         }
     }
     if (!valid) return;
@@ -234,11 +253,11 @@ __device__ __forceinline__ void dpos_dispatch(int cls, const typename DPT<FT>::t
     }
 }
 
-// FP32: two CTAs per SM (<= 128 registers); FP64: one
 template <typename FT>
-__global__ void __launch_bounds__(32 * kDposWarps, sizeof(FT) == 4 ? 2 : 1)
+__global__ void __launch_bounds__(32 * kDposWarps<FT>, sizeof(FT) == 4 ? 2 : 1)
     k_overlap2c_dpos(const __grid_constant__ DposParams<FT> P) {
-    __shared__ double part[kDposWarps][3][32];
+    constexpr int W = kDposWarps<FT>;
+    __shared__ double part[W][3][32];
     __shared__ int s_tile;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ntiles = *P.ntiles;
@@ -255,7 +274,7 @@ __global__ void __launch_bounds__(32 * kDposWarps, sizeof(FT) == 4 ? 2 : 1)
         load_geo(geo, P.posA + 3 * (size_t)b, P.posB + 3 * (size_t)b, P.scale, P.use_scale != 0);
         const FT* gs0 = P.dS + (size_t)b * P.N * P.N;
         double acc[3] = {0.0, 0.0, 0.0};
-        for (int i = warp; i < P.nitems; i += kDposWarps) {
+        for (int i = warp; i < P.nitems; i += W) {
             const Item wi = P.items[i];
             const int q = (k * P.ns + wi.sa) * P.ns + wi.sb;
             const int nrec = P.counts[q];
@@ -272,7 +291,7 @@ __global__ void __launch_bounds__(32 * kDposWarps, sizeof(FT) == 4 ? 2 : 1)
             for (int c = 0; c < 3; ++c) {
                 double s = 0.0;
 #pragma unroll
-                for (int w = 0; w < kDposWarps; ++w) s += part[w][c][lane];
+                for (int w = 0; w < W; ++w) s += part[w][c][lane];
                 if (P.dA) P.dA[3 * (size_t)b + c] = (FT)(sc * s);
                 if (P.dB) P.dB[3 * (size_t)b + c] = (FT)(-sc * s);
             }
@@ -334,10 +353,10 @@ static int launch_dpos_T(aok_plan* p, void* dA, void* dB, const void* dS, const 
     for (int i = 0; i <= p->ns; ++i) P.boff[i] = (int)p->boff[i];
     auto kern = k_overlap2c_dpos<FT>;
     int occ = 0;
-    AOK_TRY_PB(kernel_prepare((const void*)kern, 0, 32 * kDposWarps, &occ));
+    AOK_TRY_PB(kernel_prepare((const void*)kern, 0, 32 * kDposWarps<FT>, &occ));
     const int grid = std::max(1, std::min(p->max_tiles, p->num_sms * std::max(occ, 1)));
     timing_begin(p, s);
-    kern<<<grid, 32 * kDposWarps, 0, s>>>(P);
+    kern<<<grid, 32 * kDposWarps<FT>, 0, s>>>(P);
     timing_end(p, s);
     return cuda_status(cudaGetLastError(), "k_overlap2c_dpos");
 }
