@@ -248,7 +248,7 @@ int setup_moments3(aok_plan* p) {
             for (int sa = 0; sa < ns; ++sa) {
                 const int cls = canon3((int)p->ls[sa], (int)p->ls[sb], (int)p->ls[sc]).cls;
                 items.push_back(Item3{(short)sa, (short)sb, (short)sc, (short)cls, slots});
-                slots += kClass3Host[cls].D;
+                slots += kClass3Host[cls].D * (fsz == 4 ? mom_words3<float>(cls) : 1);
             }
     std::vector<Panel3> panels;
     std::vector<Out3> table;

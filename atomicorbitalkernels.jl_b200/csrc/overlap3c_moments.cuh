@@ -27,9 +27,9 @@
 // What bounds it: latency and instruction fetch.  The recursions are straight-line code run
 // once per (block, tile) by few warps, the moment sums a chain of exponentials.  777
 // elements of a 32-function basis of two elements (s to f, up to 8 primitives per shell):
-// 3,850 -> 490 us in FP64 (moments 223), 3,120 -> 489 us in FP32 (moments 182), against the
-// routine with explicit E tables per triple and run-time loops; 60 elements 2,280 -> 253 and
-// 1,880 -> 257 us.  The output alone is 31 and 16 us.
+// 3,815 -> 486 us in FP64 (moments 223), 3,120 -> 495 us in FP32, against the routine with
+// explicit E tables per triple and run-time loops; 60 elements 2,280 -> 253 and 1,880 -> 290
+// us.  The output alone is 31 and 16 us.
 // Tried: the recursions run by one warp per panel without barriers (2,600 us: one f block is
 // a long serial chain that holds up its whole panel); the moments summed in the same CTA as
 // a phase of their own (805 us).  Why the slab: stores straight from the lanes (each to its own
@@ -80,6 +80,13 @@ __host__ __device__ constexpr int class3(int l0, int l1, int l2) {
     return l0 * (l0 + 1) * (l0 + 2) / 6 + l1 * (l1 + 1) / 2 + l2;
 }
 static_assert(class3(2, 2, 2) == 9 && class3(3, 0, 0) == 10 && class3(3, 3, 3) == 19, "class order");
+// Blocks with an f shell have FP64 moments and recursions in FP32 too: rounded to FP32 at
+// each of up to nine steps, f-p-p was off by 1.1e-7 of its norm (6.5e-8 with E tables in
+// FP64), with the moments alone in FP32 by 8.1e-8.  Slots of a moment, in words of FT:
+template <typename FT>
+__host__ __device__ constexpr int mom_words3(int cls) {
+    return sizeof(FT) == 4 && cls >= class3(3, 0, 0) ? 2 : 1;
+}
 struct ClassInfo3 {
     short D, ops, parts, comps;
 };
@@ -283,8 +290,8 @@ __device__ __forceinline__ void add_rec3(const char* rec, double e, double (&par
 // by batch in its buffer (one per lane) and every lane sums them for its element; the sum
 // goes to hi[] + lo[] (FP32: runs of up to 8 triples, each run folded in with TwoSum;
 // FP64: hi[] alone).
-template <int L0, int L1, int L2, int K0, int NV, typename FT>
-__device__ __forceinline__ void moments3(const Block3<FT>& bl, int q0, int q1, char* buf, const double (&R)[3],
+template <int L0, int L1, int L2, int K0, int NV, typename FT, typename IT>
+__device__ __forceinline__ void moments3(const Block3<IT>& bl, int q0, int q1, char* buf, const double (&R)[3],
                                          FT (&hi)[NV], FT (&lo)[NV]) {
     const int lane = threadIdx.x & 31;
     constexpr int RB = rec_bytes3<FT>(NV);
@@ -360,11 +367,11 @@ __device__ __forceinline__ void moments3(const Block3<FT>& bl, int q0, int q1, c
     }
 }
 
-// The slots from K0 on, kMomSlots3 at a time, to out[32 (slot)] (the lane's column).
+// The slots from K0 on, kMomSlots3 at a time, to row out[32 (slot)] (a column per lane).
 // split: the CTA's warps take a share of the triples each and their sums meet in xbuf, added
 // in warp order by warp 0.
-template <int L0, int L1, int L2, int K0, typename FT>
-__device__ __forceinline__ void moments3_from(const Block3<FT>& bl, int n, char* buf, const double (&R)[3], FT* out,
+template <int L0, int L1, int L2, int K0, typename FT, typename IT>
+__device__ __forceinline__ void moments3_from(const Block3<IT>& bl, int n, char* buf, const double (&R)[3], FT* out,
                                               bool split, FT* xbuf) {
     constexpr int D = Prog3<L0, L1, L2, 0, 1>::D, NCH = (D + kMomSlots3 - 1) / kMomSlots3, S = (D + NCH - 1) / NCH;
     constexpr int NV = K0 + S <= D ? S : D - K0;
@@ -409,12 +416,12 @@ __device__ __forceinline__ void moments3_from(const Block3<FT>& bl, int n, char*
             bad = __double2float_rn(all - all);
         }
 #pragma unroll
-        for (int i = 0; i < NV; ++i) out[32 * (K0 + i)] = F32 ? (hi[i] + lo[i]) + bad : hi[i];
+        for (int i = 0; i < NV; ++i) out[32 * (K0 + i) + lane] = F32 ? (hi[i] + lo[i]) + bad : hi[i];
     }
     if constexpr (K0 + S < D) moments3_from<L0, L1, L2, K0 + S, FT>(bl, n, buf, R, out, split, xbuf);
 }
-template <int L0, int L1, int L2, typename FT>
-__device__ __noinline__ void moments3_call(const Block3<FT>& bl, int n, char* buf, const double (&R)[3], FT* out,
+template <int L0, int L1, int L2, typename FT, typename IT>
+__device__ __noinline__ void moments3_call(const Block3<IT>& bl, int n, char* buf, const double (&R)[3], FT* out,
                                            bool split, FT* xbuf) {
     moments3_from<L0, L1, L2, 0, FT>(bl, n, buf, R, out, split, xbuf);
 }
@@ -432,9 +439,8 @@ template <int L0, int L1, int L2, int PART, int NP, typename FT>
 __device__ __forceinline__ void transform3_slab(const FT* mom, const Geo3<FT>& g, int o0, int o1, int o2,
                                                 const Dest3<FT>& to) {
     const int lane = threadIdx.x & 31;
-    // FP32 moments of f blocks are transformed in FP64: rounded at each of up to nine steps,
-    // f-p-p was off by 1.1e-7 of its norm instead of 8.1e-8 (FP32 steps: 419 us, FP64: 482)
-    using AT = std::conditional_t<(L0 > 2), double, FT>;
+    using AT = std::conditional_t<(L0 > 2), double, FT>;  // see mom_words3
+    const AT* m = reinterpret_cast<const AT*>(mom) + lane;
     AT d01[3], d02[3], d12[3];
     if constexpr (L0 > 0) {
         const AT s01 = o0 < o1 ? AT(1) : AT(-1), s02 = o0 < o2 ? AT(1) : AT(-1), s12 = o1 < o2 ? AT(1) : AT(-1);
@@ -449,7 +455,7 @@ __device__ __forceinline__ void transform3_slab(const FT* mom, const Geo3<FT>& g
     FT* row = to.row;
     const int t0 = to.t0, t1 = to.t1, t2 = to.t2;
     const bool on = to.on;
-    transform3<L0, L1, L2, PART, NP, AT>([&](int k) { return (AT)__ldcs(mom + 32 * k); }, d01, d02, d12,
+    transform3<L0, L1, L2, PART, NP, AT>([&](int k) { return __ldcs(m + 32 * k); }, d01, d02, d12,
                                          [&](int c0, int c1, int c2, AT v) {
                                              if (on) row[c0 * t0 + c1 * t1 + c2 * t2] = (FT)v;
                                          });
@@ -520,7 +526,7 @@ template <typename FT>
 __global__ void __launch_bounds__(kThreads3, kMomCtas3) k_moments3(const __grid_constant__ Ov3Params<FT> P) {
     constexpr int W = kWarps3;
     __shared__ __align__(16) char recbuf[W][kRecBytes3];
-    __shared__ FT xbuf[(W - 1) * kMomSlots3 * (sizeof(FT) == 4 ? 64 : 32)];
+    __shared__ __align__(16) FT xbuf[(W - 1) * kMomSlots3 * (sizeof(FT) == 4 ? 64 : 32)];
     __shared__ unsigned claim;
     pdl_wait();  // launched programmatically after k_overlap3c or the last round: the bins, the prep's order and the
                  // buffers are complete past here
@@ -574,14 +580,16 @@ __global__ void __launch_bounds__(kThreads3, kMomCtas3) k_moments3(const __grid_
             }
             const int n = bl.n[0] * bl.n[1] * bl.n[2];
             if (n == 0) continue;  // k_transform3 writes zeros
-            FT* out = P.mom + ((size_t)tile * P.slots + wi.moff) * 32 + lane;
+            FT* out = P.mom + ((size_t)tile * P.slots + wi.moff) * 32;
             switch (wi.cls) {
 #define AOK_X(a, b, c, np)                                                                 \
     case class3(a, b, c):                                                                  \
         if constexpr (a + b + c <= 2)                                                      \
             moments3_from<a, b, c, 0, FT>(bl, n, recbuf[warp], R, out, split, xbuf);       \
-        else                                                                               \
+        else if constexpr (a <= 2)                                                         \
             moments3_call<a, b, c, FT>(bl, n, recbuf[warp], R, out, split, xbuf);          \
+        else                                                                               \
+            moments3_call<a, b, c, double>(bl, n, recbuf[warp], R, (double*)out, split, (double*)xbuf); \
         break;
                 AOK_CLASSES3(AOK_X)
                 default: break;
@@ -629,9 +637,10 @@ __global__ void __launch_bounds__(kTrThreads3<FT>, kTrCtas3<FT>) k_transform3(co
         const int key = td.x, ga = key / (P.NZ * P.NZ), gb = (key / P.NZ) % P.NZ, gc = key % P.NZ;
         const bool on = lane < pn.nsa;
         const int sa = pn.sa0 + (on ? lane : 0), la = P.l[sa], lb = P.l[pn.sb], lc = P.l[pn.sc];
-        const ClassInfo3 ci = kClass3[canon3(la, lb, lc).cls];
+        const int cls = canon3(la, lb, lc).cls;
+        const ClassInfo3 ci = kClass3[cls];
         const bool zero = P.pn[ga * P.ns + sa] * P.pn[gb * P.ns + pn.sb] * P.pn[gc * P.ns + pn.sc] == 0;
-        const int t0 = on ? (zero ? 1 : ci.parts) : 0, s0 = on ? ncart(la) * ncart(lb) * ncart(lc) : 0, m0 = on ? ci.D : 0;
+        const int t0 = on ? (zero ? 1 : ci.parts) : 0, s0 = on ? ncart(la) * ncart(lb) * ncart(lc) : 0, m0 = on ? ci.D * mom_words3<FT>(cls) : 0;
         int t = t0, so = s0, m = m0;
 #pragma unroll
         for (int o = 1; o < kPanelItems3; o <<= 1) {
@@ -678,7 +687,7 @@ __global__ void __launch_bounds__(kTrThreads3<FT>, kTrCtas3<FT>) k_transform3(co
         const int lb = P.l[pn.sb], lc = P.l[pn.sc], NB = ncart(lb), NC = ncart(lc);
         const int lanes = 32 / pn.passes, rowlen = (pn.comps + 1) | 1;
         const int nt = pn.pass * lanes < U.cnt ? U.t[pn.nsa] : 0;  // a partial tile may not reach this pass
-        const FT* tile_mom = P.mom + (size_t)U.tile * P.slots * 32 + lane;
+        const FT* tile_mom = P.mom + (size_t)U.tile * P.slots * 32;
         FT* row = slab + (size_t)(lane & (lanes - 1)) * rowlen;
         if (warp == 0 && lane < lanes) row[pn.comps] = FT(0);
         for (;;) {
