@@ -296,6 +296,7 @@ __device__ __forceinline__ EvalSmem<FT> eval_smem(unsigned char* raw, int ntab, 
 
 template <typename FT, int L, bool GRAD>
 __global__ void __launch_bounds__(kEvalThreads) k_evaluate(const __grid_constant__ EvalParams P) {
+    pdl_wait();  // launched programmatically: its inputs and buffers are free past here
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int nY = (L + 1) * (L + 1);
     const int ntab = P.nRad * P.K * P.NZ;
@@ -413,6 +414,7 @@ __device__ __forceinline__ void emit_block(FT R, FT dR, FT ux, FT uy, FT uz, FT 
 
 template <typename FT, int L, bool GRAD, bool BLK = false>
 __global__ void __launch_bounds__(kEvalThreads) k_evaluate_reg(const __grid_constant__ EvalRegParams Q) {
+    pdl_wait();  // launched programmatically: its inputs and buffers are free past here
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const EvalParams& P = Q.E;
     constexpr int nY = (L + 1) * (L + 1);
@@ -699,6 +701,7 @@ __host__ __device__ constexpr size_t epb_acc_words(int nRad, int K, int NZ) { re
 // k_evaluate_reg), so a warp's shared memory holds only gg and f(r).
 template <typename FT, int L, bool RAD = false, bool REG = false>
 __global__ void __launch_bounds__(256, 4) k_evaluate_pbs(const __grid_constant__ EpbParams Q) {
+    pdl_wait();  // launched programmatically: its inputs and buffers are free past here
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int nY = (L + 1) * (L + 1);
     const EvalParams& P = Q.E;
@@ -959,6 +962,7 @@ __global__ void __launch_bounds__(kEpbRedThreads) k_epb_reduce(FT* __restrict__ 
                                                                const double* __restrict__ partial,
                                                                const FT* __restrict__ zeta, const FT* __restrict__ D,
                                                                int nRad, int K, int nout, int nunits, int ucap) {
+    pdl_wait();  // launched programmatically after k_evaluate_pbs: its rows are complete past here
     __shared__ double ws[kEpbRedThreads / 32];
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int kind = t / nout, o = t - kind * nout;  // o = slot + nRad K species
@@ -997,15 +1001,14 @@ __global__ void __launch_bounds__(kEpbRedThreads) k_epb_reduce(FT* __restrict__ 
 static int launch_epb_reduce(aok_orbitals* o, void* dD, void* dzeta, const EpbParams& Q, cudaStream_t s) {
     const int nout = (int)(o->nRad * o->K * o->NZ), nunits = Q.nrows;
     const int nRad = (int)o->nRad, K = (int)o->K;
-    if (o->prec == AOK_PREC_F64)
-        k_epb_reduce<double><<<2 * nout, kEpbRedThreads, 0, s>>>((double*)dD, (double*)dzeta, Q.partial,
-                                                                  (const double*)Q.E.zeta, (const double*)Q.E.D,
-                                                                  nRad, K, nout, nunits, Q.ucap);
-    else
-        k_epb_reduce<float><<<2 * nout, kEpbRedThreads, 0, s>>>((float*)dD, (float*)dzeta, Q.partial,
-                                                                 (const float*)Q.E.zeta, (const float*)Q.E.D, nRad,
-                                                                 K, nout, nunits, Q.ucap);
-    return cuda_status(cudaGetLastError(), "k_epb_reduce");
+    const dim3 grid(2 * nout), block(kEpbRedThreads);
+    const cudaError_t e =
+        o->prec == AOK_PREC_F64
+            ? launch_pdl(k_epb_reduce<double>, grid, block, 0, s, (double*)dD, (double*)dzeta, (const double*)Q.partial,
+                         (const double*)Q.E.zeta, (const double*)Q.E.D, nRad, K, nout, nunits, Q.ucap)
+            : launch_pdl(k_epb_reduce<float>, grid, block, 0, s, (float*)dD, (float*)dzeta, (const double*)Q.partial,
+                         (const float*)Q.E.zeta, (const float*)Q.E.D, nRad, K, nout, nunits, Q.ucap);
+    return cuda_status(e, "k_epb_reduce");
 }
 
 template <typename FT>
@@ -1091,8 +1094,7 @@ static int launch_eval_L(aok_orbitals* o, EvalParams& P, bool grad, bool pb, cud
     int occ = 0;
     AOK_TRY_PB(kernel_prepare((const void*)k, smem, kEvalThreads, &occ));
     grid = std::max(1, std::min(grid, o->num_sms * std::max(occ, 1)));
-    k<<<grid, kEvalThreads, smem, s>>>(P);
-    return cuda_status(cudaGetLastError(), "k_evaluate");
+    return cuda_status(launch_pdl_at((const void*)k, grid, kEvalThreads, smem, s, &P), "k_evaluate");
 }
 
 template <typename FT>
@@ -1192,8 +1194,7 @@ static int launch_eval_reg_L(aok_orbitals* o, const EvalParams& P, bool grad, cu
     AOK_TRY_PB(kernel_prepare(k, smem, kEvalThreads, &occ));
     const int grid = (int)std::max<int64_t>(
         1, std::min<int64_t>((P.nX + kEvalThreads - 1) / kEvalThreads, (int64_t)o->num_sms * std::max(occ, 1)));
-    void* args[] = {&Q};
-    return cuda_status(cudaLaunchKernel(k, dim3(grid), dim3(kEvalThreads), args, smem, s), "k_evaluate_reg");
+    return cuda_status(launch_pdl_at(k, grid, kEvalThreads, smem, s, &Q), "k_evaluate_reg");
 }
 
 template <typename FT>
@@ -1254,8 +1255,7 @@ static int launch_epb_kernel(aok_orbitals* o, const void* k, EpbParams& Q, size_
     const int grid = (int)std::max<int64_t>(
         1, std::min<int64_t>(std::min<int64_t>(want, (int64_t)o->num_sms * std::max(occ, 1)), Q.ucap));
     Q.nrows = grid;
-    void* args[] = {&Q};
-    return cuda_status(cudaLaunchKernel(k, dim3(grid), dim3(32 * nw), args, smem, s), what);
+    return cuda_status(launch_pdl_at(k, grid, 32 * nw, smem, s, &Q), what);
 }
 
 template <typename FT, int L>
