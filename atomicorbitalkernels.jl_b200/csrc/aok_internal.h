@@ -206,6 +206,10 @@ struct BinBufs {
     // the second launch programmatically after the first: where the binning is alone on the
     // device (beside record preparations on the side stream it loses more than the launch)
     bool pdl = false;
+    // the first launch programmatically after the caller's previous work: 2 us a call (257 pairs
+    // 22.6 -> 20.5 us, 65,536 175.7 -> 173.9); not beside the position pullback's short record
+    // preparation (8,191 pairs FP32 69.0 -> 71.7 us)
+    bool first_pdl = true;
 };
 constexpr int kBinMaxBlocksHost = 512;
 int launch_bin_into(const BinBufs& bb, const int64_t* sidxA, const int64_t* sidxB, int64_t B, int NZ,

@@ -425,7 +425,8 @@ __global__ void __launch_bounds__(kBinThreads) k_bin_count(const int64_t* __rest
                                                             int* __restrict__ err, void* zero3, void* zero3b,
                                                             int zero3_bytes) {
     __shared__ int hist[kMaxPairs];
-    pdl_trigger();  // the scatter may launch now (it waits for this grid's end)
+    pdl_wait();     // the first launch of a call, programmatically after whatever came before
+    pdl_trigger();  // past that: the scatter, which reads the indices at once, may launch now
     for (int k = threadIdx.x; k < np; k += blockDim.x) hist[k] = 0;
     __syncthreads();
     const int c0 = blockIdx.x * chunk, c1 = min(B, c0 + chunk);
@@ -581,7 +582,8 @@ __global__ void k_bin_identity(int B, int np, int* __restrict__ perm, int4* __re
                                int* __restrict__ ntiles, int* __restrict__ tbase, unsigned* __restrict__ counter,
                                const int64_t* __restrict__ sidxA, const int64_t* __restrict__ sidxB,
                                const int64_t* __restrict__ sidxC, int NZ, int* __restrict__ err) {
-    pdl_trigger();  // a programmatic successor may launch now (it waits for this grid's end)
+    pdl_wait();     // the first launch of a call, programmatically after whatever came before
+    pdl_trigger();  // past that: a programmatic successor may launch now (it waits for this grid's end)
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     const int nt = (B + kTileB - 1) / kTileB;
     if (b < B && (sidxA || sidxB || sidxC)) (void)pair_key(sidxA, sidxB, sidxC, b, B, NZ, err);
@@ -804,14 +806,20 @@ int launch_bin3_into(const BinBufs& bb, const int64_t* sidxA, const int64_t* sid
     const int maxb = std::min(kBinMaxBlocks, std::max(128, 16384 / np));
     const int chunk = (int)std::max<int64_t>(512, (B + maxb - 1) / maxb);
     const int nblk = (int)((B + chunk - 1) / chunk);
+    auto first = [&](auto kern, dim3 grid, dim3 block, auto... args) {
+        if (bb.first_pdl) return launch_pdl(kern, grid, block, 0, s, args...);
+        kern<<<grid, block, 0, s>>>(args...);
+        return cudaGetLastError();
+    };
     if (NZ == 1 || (!sidxA && !sidxB && !sidxC)) {
-        k_bin_identity<<<(int)((std::max<int64_t>(B, np + 1) + 255) / 256), 256, 0, s>>>(
-            (int)B, np, bb.perm, bb.tiles, bb.ntiles, bb.tbase, bb.counter, sidxA, sidxB, sidxC, NZ, bb.err);
-        return cuda_status(cudaGetLastError(), "k_bin_identity");
+        return cuda_status(first(k_bin_identity, dim3((unsigned)((std::max<int64_t>(B, np + 1) + 255) / 256)), dim3(256),
+                                 (int)B, np, bb.perm, bb.tiles, bb.ntiles, bb.tbase, bb.counter, sidxA, sidxB, sidxC,
+                                 NZ, bb.err),
+                           "k_bin_identity");
     }
-    k_bin_count<<<nblk, kBinThreads, 0, s>>>(sidxA, sidxB, sidxC, (int)B, NZ, np, chunk, bb.blockhist, bb.err,
-                                             bb.zero3, bb.zero3b, bb.zero3_bytes);
-    AOK_TRY_ST(cuda_status(cudaGetLastError(), "k_bin_count"));
+    AOK_TRY_ST(cuda_status(first(k_bin_count, dim3(nblk), dim3(kBinThreads), sidxA, sidxB, sidxC, (int)B, NZ, np, chunk,
+                                 bb.blockhist, bb.err, bb.zero3, bb.zero3b, bb.zero3_bytes),
+                           "k_bin_count"));
     if (bb.pdl)
         return cuda_status(launch_pdl(k_bin_scatter, dim3(nblk), dim3(kBinThreads), 0, s, sidxA, sidxB, sidxC, (int)B, NZ,
                                       np, chunk, (const int*)bb.blockhist, bb.perm, bb.tiles, bb.ntiles, bb.tbase,

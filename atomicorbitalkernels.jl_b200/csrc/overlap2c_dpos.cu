@@ -383,6 +383,7 @@ int launch_overlap2c_dpos(aok_plan* p, void* dA, void* dB, const void* dS, const
     AOK_TRY_PB(cuda_status(cudaEventRecord(p->ev_join, p->side), "cudaEventRecord"));
     ++p->gen;  // the plan's bins change
     BinBufs bb{p->d_perm, p->d_tiles, p->d_ntiles, p->d_tbase, p->d_counter, p->d_blockhist, p->d_err};
+    bb.first_pdl = false;
     bb.zero3 = dA;
     bb.zero3b = dB;
     bb.zero3_bytes = p->prec == AOK_PREC_F64 ? 8 : 4;
