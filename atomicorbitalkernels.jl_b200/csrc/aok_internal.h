@@ -228,7 +228,9 @@ int ensure_pb_buffers(aok_plan* p);
 int launch_overlap2c_dpos(aok_plan* p, void* dA, void* dB, const void* dS, const void* zeta, const void* coef,
                           const int64_t* sidxA, const int64_t* sidxB, const void* posA, const void* posB, int64_t B,
                           double lengthscale, cudaStream_t s);
-int launch_prep_pb(aok_plan* p, const void* zeta, const void* coef, int keep_absent, cudaStream_t s);
+// counter: a work counter zeroed on the way, or nullptr
+int launch_prep_pb(aok_plan* p, const void* zeta, const void* coef, int keep_absent, cudaStream_t s,
+                   unsigned* counter = nullptr);
 // pdl: launched with programmatic serialisation after the binning (or the record packing) on
 // the same stream
 int launch_overlap2c(aok_plan* p, void* out, const void* posA, const void* posB, int64_t B,

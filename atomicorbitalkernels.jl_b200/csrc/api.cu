@@ -516,17 +516,20 @@ int aok_overlap2c_rrule(aok_plan* p, void* out, const void* zeta, const void* D,
         AOK_TRY(cuda_status(cudaEventCreateWithFlags(&p->ev_pb, cudaEventDisableTiming), "cudaEventCreate"));
     p->basis_set = false;
     void* coef = p->d_coef_scratch;
-    // side stream: coef, the forward records, then (while the overlap kernel runs) the pullback records
+    // this stream: coef, the forward records and the overlap kernel, the longest chain; side
+    // stream: the bins, then the pullback records, beside the packing.  (The overlap kernel's
+    // CTAs hold every register, so records prepared after the packing kept it from starting.)
     AOK_TRY(cuda_status(cudaEventRecord(p->ev_fork, s), "cudaEventRecord"));
     AOK_TRY(cuda_status(cudaStreamWaitEvent(p->side, p->ev_fork, 0), "cudaStreamWaitEvent"));
-    AOK_TRY(launch_compile_coef(p, coef, zeta, D, p->side));
-    AOK_TRY(launch_prep2c(p, zeta, coef, p->side, true));
+    AOK_TRY(launch_compile_coef(p, coef, zeta, D, s));
+    AOK_TRY(cuda_status(cudaEventRecord(p->ev_fork, s), "cudaEventRecord"));
+    AOK_TRY(launch_bin(p, sidxA, sidxB, B, p->side));
     AOK_TRY(cuda_status(cudaEventRecord(p->ev_join, p->side), "cudaEventRecord"));
-    // the pullback kernel's work counter (the forward kernel uses the first one)
-    AOK_TRY(cuda_status(cudaMemsetAsync(p->d_counter + 1, 0, sizeof(unsigned), p->side), "cudaMemsetAsync"));
-    AOK_TRY(launch_prep_pb(p, zeta, coef, 0, p->side));
+    AOK_TRY(cuda_status(cudaStreamWaitEvent(p->side, p->ev_fork, 0), "cudaStreamWaitEvent"));
+    // and the pullback kernel's work counter (the forward kernel uses the first one)
+    AOK_TRY(launch_prep_pb(p, zeta, coef, 0, p->side, p->d_counter + 1));
     AOK_TRY(cuda_status(cudaEventRecord(p->ev_pb, p->side), "cudaEventRecord"));
-    AOK_TRY(launch_bin(p, sidxA, sidxB, B, s));
+    AOK_TRY(launch_prep2c(p, zeta, coef, s, true));
     AOK_TRY(cuda_status(cudaStreamWaitEvent(s, p->ev_join, 0), "cudaStreamWaitEvent"));
     AOK_TRY(launch_overlap2c(p, out, posA, posB, B, lengthscale, s));
     p->rkey = aok_plan::RruleKey{zeta, D, posA, posB, sidxA, sidxB, B, lengthscale};

@@ -7,7 +7,8 @@
 
 namespace aok {
 
-int launch_prep_pb(aok_plan* p, const void* zeta, const void* coef, int keep_absent, cudaStream_t s) {
+int launch_prep_pb(aok_plan* p, const void* zeta, const void* coef, int keep_absent, cudaStream_t s,
+                   unsigned* counter) {
     ++p->gen;  // the pullback records change
     const int n = (int)(p->NZ * p->NZ * p->ns * p->ns);
     const int bl = (n + kPrepPbWarps - 1) / kPrepPbWarps;
@@ -15,11 +16,11 @@ int launch_prep_pb(aok_plan* p, const void* zeta, const void* coef, int keep_abs
     if (p->prec == AOK_PREC_F64)
         k_prep_pb<double><<<bl, 32 * kPrepPbWarps, sm, s>>>(
             (PBd*)p->d_pb_rec, p->d_pb_counts, (const double*)zeta, (const double*)coef, (int)p->ns, (int)p->K,
-            (int)p->NZ, keep_absent);
+            (int)p->NZ, keep_absent, counter);
     else
         k_prep_pb<float><<<bl, 32 * kPrepPbWarps, sm, s>>>(
             (PBf*)p->d_pb_rec, p->d_pb_counts, (const float*)zeta, (const float*)coef, (int)p->ns, (int)p->K,
-            (int)p->NZ, keep_absent);
+            (int)p->NZ, keep_absent, counter);
     return cuda_status(cudaGetLastError(), "k_prep_pb");
 }
 

@@ -101,8 +101,9 @@ constexpr int kPrepPbWarps = 4;
 template <typename FT>
 __global__ void __launch_bounds__(32 * kPrepPbWarps)
     k_prep_pb(typename PBT<FT>::type* __restrict__ rec, int4* __restrict__ counts, const FT* __restrict__ zeta,
-              const FT* __restrict__ coef, int ns, int K, int NZ, int keep_absent) {
+              const FT* __restrict__ coef, int ns, int K, int NZ, int keep_absent, unsigned* __restrict__ counter) {
     extern __shared__ unsigned char flags_raw[];  // [warp][4][K]: nzA, lsA, nzB, lsB
+    if (counter && blockIdx.x == 0 && threadIdx.x == 0) *counter = 0u;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int q = blockIdx.x * kPrepPbWarps + warp;
     if (q >= NZ * NZ * ns * ns) return;
