@@ -248,7 +248,7 @@ int setup_moments3(aok_plan* p) {
             for (int sa = 0; sa < ns; ++sa) {
                 const int cls = canon3((int)p->ls[sa], (int)p->ls[sb], (int)p->ls[sc]).cls;
                 items.push_back(Item3{(short)sa, (short)sb, (short)sc, (short)cls, slots});
-                slots += kClass3Host[cls].D * (fsz == 4 ? mom_words3<float>(cls) : 1);
+                slots += kClass3Host[cls].D;
             }
     std::vector<Panel3> panels;
     std::vector<Out3> table;
@@ -296,7 +296,7 @@ int setup_moments3(aok_plan* p) {
     // moments are kept for at most kMoments3 bytes of tiles at a time (in the L2 cache); a
     // larger batch goes through in rounds.  One tile always fits: the panel schedule of the
     // plan bounds N to about 120 (64 shells of 83 functions, FP64: 70 MB).
-    const int64_t most = (p->max_batch + 31) / 32 + bin_keys_max(p->NZ) + 1, tile = (int64_t)slots * 32 * (int64_t)fsz;
+    const int64_t most = (p->max_batch + 31) / 32 + bin_keys_max(p->NZ) + 1, tile = (int64_t)slots * 32 * (int64_t)sizeof(double);
     p->round3 = (int)std::max<int64_t>(1, std::min(most, kMoments3 / tile));
     p->nrounds3 = (int)((most + p->round3 - 1) / p->round3);
     p->npanels3 = (int)panels.size();

@@ -27,8 +27,8 @@
 // What bounds it: latency and instruction fetch.  The recursions are straight-line code run
 // once per (block, tile) by few warps, the moment sums a chain of exponentials.  777
 // elements of a 32-function basis of two elements (s to f, up to 8 primitives per shell):
-// 3,815 -> 486 us in FP64 (moments 223), 3,120 -> 495 us in FP32, against the routine with
-// explicit E tables per triple and run-time loops; 60 elements 2,280 -> 253 and 1,880 -> 290
+// 3,815 -> 472 us in FP64 (moments 210), 3,120 -> 444 us in FP32, against the routine with
+// explicit E tables per triple and run-time loops; 60 elements 2,280 -> 244 and 1,880 -> 225
 // us.  The output alone is 31 and 16 us.
 // Tried: the recursions run by one warp per panel without barriers (2,600 us: one f block is
 // a long serial chain that holds up its whole panel); the moments summed in the same CTA as
@@ -39,7 +39,6 @@
 
 #include <algorithm>
 #include <cstring>
-#include <type_traits>
 
 #include "aok_internal.h"
 #include "moment3c.cuh"
@@ -54,20 +53,16 @@ constexpr int64_t kMoments3 = 256 << 20;
 constexpr int kPanelItems3 = 16;     // A shells of a panel
 constexpr int kRecBytes3 = 3072;     // record buffer of a warp (k_moments3)
 constexpr int kMomSlots3 = 28;       // moments summed at a time (registers)
-// k_transform3 (<= 168 registers): FP32 two CTAs of 6 warps per SM, FP64 one of 12, whose
-// slab holds the larger blocks in fewer element groups (577 -> 500 us for 777 elements of a
-// 32-function basis; FP32 gained nothing from it, 415 -> 419 us).  Shared memory: geometry
-// and slab.
-template <typename FT> constexpr int kTrThreads3 = sizeof(FT) == 4 ? 192 : 384;
-template <typename FT> constexpr int kTrCtas3 = sizeof(FT) == 4 ? 2 : 1;
-template <typename FT> constexpr int kTrSmem3 = (sizeof(FT) == 4 ? 110 : 222) * 1024;
+// k_transform3 (<= 168 registers): one CTA of 12 warps per SM, whose slab holds the larger
+// blocks in fewer element groups than two CTAs of 6 warps would (777 elements of a
+// 32-function basis: FP64 500 against 577 us, FP32 484 against 527).  Shared memory:
+// geometry and slab.
+constexpr int kTrThreads3 = 384;
+constexpr int kTrSmem3 = 222 * 1024;
 
 // Record of a primitive triple of a class with D moments: the exponent's three
-// coefficients (FP64; times log2(e) for FP32) and the moments' factors w mono_m.
-template <typename FT>
-__host__ __device__ constexpr int rec_bytes3(int nv) {
-    return ((24 + (sizeof(FT) == 4 ? 4 * (nv + (nv & 1)) : 8 * nv)) + 15) / 16 * 16;
-}
+// coefficients (times log2(e) for ex2_neg3) and the moments' factors w mono_m.
+__host__ __device__ constexpr int rec_bytes3(int nv) { return (24 + 8 * nv + 15) / 16 * 16; }
 
 // Canonical classes L0 >= L1 >= L2, in the order of class3().
 #define AOK_CLASSES3(X) \
@@ -80,13 +75,16 @@ __host__ __device__ constexpr int class3(int l0, int l1, int l2) {
     return l0 * (l0 + 1) * (l0 + 2) / 6 + l1 * (l1 + 1) / 2 + l2;
 }
 static_assert(class3(2, 2, 2) == 9 && class3(3, 0, 0) == 10 && class3(3, 3, 3) == 19, "class order");
-// Blocks with an f shell have FP64 moments and recursions in FP32 too: rounded to FP32 at
-// each of up to nine steps, f-p-p was off by 1.1e-7 of its norm (6.5e-8 with E tables in
-// FP64), with the moments alone in FP32 by 8.1e-8.  Slots of a moment, in words of FT:
+// Moments and recursions are FP64 in both precisions.  With FP32 sums (runs of 8 triples
+// folded with TwoSum) and FP32 recursions up to d, p-p-p, d-p-p, d-d-p and d-d-d were off by up
+// to 1.3 times as much as with E tables (norm of the block, d-d-p of two primitives per shell:
+// 1.03e-7 against 8.2e-8); so they are off by 3e-8 to 4.7e-8 in every class, and 777 elements
+// take 444 us (FP32 sums and recursions: 488).  Up to d FP32 takes its exponentials from ex2
+// (rounding of the result apart, the error that is left); with FP64 ones every class is at
+// 2.5e-8 to 3.6e-8, but 777 elements take 484 us and 1,500 take 824 (758 with ex2).  Blocks
+// with an f shell have them in FP64, as their E tables do.
 template <typename FT>
-__host__ __device__ constexpr int mom_words3(int cls) {
-    return sizeof(FT) == 4 && cls >= class3(3, 0, 0) ? 2 : 1;
-}
+__host__ __device__ constexpr bool fast_exp3(int l0) { return sizeof(FT) == 4 && l0 <= 2; }
 struct ClassInfo3 {
     short D, ops, parts, comps;
 };
@@ -132,12 +130,12 @@ struct Panel3 {
     int comps;               // slab elements of a batch element: sum of NA NB NC
     short passes, pass;      // the slab holds 32 / passes elements: this panel's are those of pass
     int tab, nout;           // the panel's output elements: entries [tab, tab + nout) of the table
-    int moff;                // first moment slot
+    int moff;                // first moment
 };
 // One block (shell triple) for the moment kernel.
 struct Item3 {
     short sa, sb, sc, cls;
-    int moff;                // first moment slot
+    int moff;                // first moment
 };
 // Output element of a panel: the slab elements that the aliased layout adds into it (at
 // most 2 x 2; the rest name the row's zero element, index comps) and its offset from the panel's first element.
@@ -156,7 +154,7 @@ struct __align__(16) Geo3 {
 // Slab elements (of FT) that a CTA has.
 template <typename FT>
 __host__ __device__ constexpr int slab_room3() {
-    return (kTrSmem3<FT> - 2 * (int)sizeof(Geo3<FT>)) / (int)sizeof(FT);
+    return (kTrSmem3 - 2 * (int)sizeof(Geo3<FT>)) / (int)sizeof(FT);
 }
 
 // The pair differences A - B, A - C, B - C in FP64 (exact for FP32 positions); positions
@@ -204,21 +202,21 @@ struct Slots3 {
         constexpr int a = kMono.a[K0 + J], b = kMono.b[K0 + J], g = kMono.g[K0 + J], d = kMono.d[K0 + J];
         return (pa[a] * pb[b]) * (pg[g] * ph[d]);
     }
-    template <typename FT, int... J>
-    static __device__ __forceinline__ void fill(FT* v, const double* pa, const double* pb, const double* pg,
+    template <int... J>
+    static __device__ __forceinline__ void fill(double* v, const double* pa, const double* pb, const double* pg,
                                                 const double* ph, Seq<J...>) {
-        ((v[J] = (FT)one<J>(pa, pb, pg, ph)), ...);
+        ((v[J] = one<J>(pa, pb, pg, ph)), ...);
     }
 };
 
-// Record of the triple (a, b, c) with coefficients ca, cb, cc (FP64 arithmetic):
-// moment slots [K0, K0 + NV) of the class.
-template <int L0, int L1, int L2, int K0, int NV, typename FT>
+// Record of the triple (a, b, c) with coefficients ca, cb, cc: moment slots [K0, K0 + NV)
+// of the class.
+template <int L0, int L1, int L2, int K0, int NV, bool EX2>
 __device__ __forceinline__ void fill_rec3(char* rec, double ca, double cb, double cc, double a, double b, double c) {
     using PR = Prog3<L0, L1, L2, 0, 1>;
     const double q = a + b + c, iq = 1.0 / q, x = 3.14159265358979323846 * iq;
-    const double l2e = sizeof(FT) == 4 ? 1.4426950408889634074 : 1.0;
     double* k = reinterpret_cast<double*>(rec);
+    const double l2e = EX2 ? 1.4426950408889634074 : 1.0;
     k[0] = a * b * iq * l2e;
     k[1] = a * c * iq * l2e;
     k[2] = b * c * iq * l2e;
@@ -233,16 +231,13 @@ __device__ __forceinline__ void fill_rec3(char* rec, double ca, double cb, doubl
     for (int i = 1; i < PR::MG; ++i) pg[i] = pg[i - 1] * (c * iq);
 #pragma unroll
     for (int i = 1; i <= PR::n / 2; ++i) ph[i] = ph[i - 1] * (0.5 * iq);
-    FT* v = reinterpret_cast<FT*>(rec + 24);
-    Slots3<L0, L1, L2, K0>::fill(v, pa, pb, pg, ph, MakeSeq<NV>{});
-    if (sizeof(FT) == 4 && (NV & 1)) v[NV] = FT(0);
+    Slots3<L0, L1, L2, K0>::fill(k + 3, pa, pb, pg, ph, MakeSeq<NV>{});
 }
 
 // 2^-x with x given in FP64 (log2 units): the integer part goes into the exponent field,
 // the fraction (|f| <= 1/2, so one rounding to FP32 costs 2^-26 of the result) through
-// ex2.  One FP64 -> FP32 conversion, where a hi + lo split of x takes three.  x is cut off
-// at 200 through its high word, and 2^-n is 0 from n = 127 on; an infinite or NaN distance
-// is put back by the caller.
+// ex2.  x is cut off at 200 through its high word, and 2^-n is 0 from n = 127 on; an
+// infinite or NaN distance is put back by the caller.
 __device__ __forceinline__ float ex2_neg3(double x) {
     const double magic = 6755399441055744.0;  // 1.5 * 2^52: the sum's low word is round(x)
     x = __hiloint2double(min(__double2hiint(x), 0x40690000), __double2loint(x));
@@ -250,31 +245,15 @@ __device__ __forceinline__ float ex2_neg3(double x) {
     const float f = __double2float_rn(x - (t - magic));
     return ex2_approx(-f) * __int_as_float(min(max(127 - __double2loint(t), 0), 255) << 23);
 }
-
 // e^{-arg} of one record for the lane's squared distances.
-__device__ __forceinline__ float rec_exp3(const char* rec, double R0, double R1, double R2, float) {
+template <bool EX2>
+__device__ __forceinline__ double rec_exp3(const char* rec, double R0, double R1, double R2) {
     const double2 k = *reinterpret_cast<const double2*>(rec);
     const double k2 = *reinterpret_cast<const double*>(rec + 16);
-    return ex2_neg3(fma(k2, R2, fma(k.y, R1, k.x * R0)));
-}
-__device__ __forceinline__ double rec_exp3(const char* rec, double R0, double R1, double R2, double) {
-    const double2 k = *reinterpret_cast<const double2*>(rec);
-    const double k2 = *reinterpret_cast<const double*>(rec + 16);
+    if (EX2) return (double)ex2_neg3(fma(k2, R2, fma(k.y, R1, k.x * R0)));
     return exp(-fma(k2, R2, fma(k.y, R1, k.x * R0)));
 }
-// Adds e times one record's factors.  part: FP32 pairs of slots, FP64 slots.
-template <int NV>
-__device__ __forceinline__ void add_rec3(const char* rec, float e, float2 (&part)[(NV + 1) / 2]) {
-    constexpr int NP = (NV + 1) / 2;
-    const float2 ee = make_float2(e, e);
-    part[0] = __ffma2_rn(ee, *reinterpret_cast<const float2*>(rec + 24), part[0]);
-#pragma unroll
-    for (int i = 1; i < NP; i += 2) {
-        const float4 q = *reinterpret_cast<const float4*>(rec + 24 + 8 * i);
-        part[i] = __ffma2_rn(ee, make_float2(q.x, q.y), part[i]);
-        if (i + 1 < NP) part[i + 1] = __ffma2_rn(ee, make_float2(q.z, q.w), part[i + 1]);
-    }
-}
+// Adds e times one record's factors.
 template <int NV>
 __device__ __forceinline__ void add_rec3(const char* rec, double e, double (&part)[NV]) {
     part[0] = fma(e, *reinterpret_cast<const double*>(rec + 24), part[0]);
@@ -287,27 +266,20 @@ __device__ __forceinline__ void add_rec3(const char* rec, double e, double (&par
 }
 
 // Moment slots [K0, K0 + NV) of a block's triples [q0, q1): the warp builds records batch
-// by batch in its buffer (one per lane) and every lane sums them for its element; the sum
-// goes to hi[] + lo[] (FP32: runs of up to 8 triples, each run folded in with TwoSum;
-// FP64: hi[] alone).
-template <int L0, int L1, int L2, int K0, int NV, typename FT, typename IT>
-__device__ __forceinline__ void moments3(const Block3<IT>& bl, int q0, int q1, char* buf, const double (&R)[3],
-                                         FT (&hi)[NV], FT (&lo)[NV]) {
+// by batch in its buffer (one per lane) and every lane sums them for its element.
+template <int L0, int L1, int L2, int K0, int NV, typename FT>
+__device__ __forceinline__ void moments3(const Block3<FT>& bl, int q0, int q1, char* buf, const double (&R)[3],
+                                         double (&sum)[NV]) {
     const int lane = threadIdx.x & 31;
-    constexpr int RB = rec_bytes3<FT>(NV);
-    constexpr int NB = kRecBytes3 / RB >= 32 ? 32 : kRecBytes3 / RB / 8 * 8;
+    constexpr int RB = rec_bytes3(NV);
+    constexpr bool EX2 = fast_exp3<FT>(L0);
+    constexpr int NB = kRecBytes3 / RB >= 32 ? 32 : kRecBytes3 / RB;
     static_assert(NB >= 8, "record buffer");
-    constexpr bool F32 = sizeof(FT) == 4;
-    constexpr int NP = F32 ? (NV + 1) / 2 : NV;
-    using Acc = std::conditional_t<F32, float2, double>;
     const int n12 = bl.n[1] * bl.n[2], n2 = bl.n[2];
     const float f12 = 1.f / (float)n12, f2 = 1.f / (float)n2;
     const double R0 = R[pair3(bl.o0, bl.o1)], R1 = R[pair3(bl.o0, bl.o2)], R2 = R[pair3(bl.o1, bl.o2)];
-    Acc part[NP];
 #pragma unroll
-    for (int i = 0; i < NP; ++i) part[i] = Acc{};
-#pragma unroll
-    for (int i = 0; i < NV; ++i) hi[i] = lo[i] = FT(0);
+    for (int i = 0; i < NV; ++i) sum[i] = 0.0;
 #pragma unroll 1
     for (int qb = q0; qb < q1; qb += NB) {
         const int m = min(NB, q1 - qb);
@@ -321,108 +293,69 @@ __device__ __forceinline__ void moments3(const Block3<IT>& bl, int q0, int q1, c
             int j = (int)((float)r * f2), k = r - j * n2;
             j += k >= n2 ? 1 : k < 0 ? -1 : 0;
             k = r - j * n2;
-            fill_rec3<L0, L1, L2, K0, NV, FT>(buf + lane * RB, (double)bl.c[0][i], (double)bl.c[1][j],
-                                              (double)bl.c[2][k], (double)bl.z[0][i], (double)bl.z[1][j],
-                                              (double)bl.z[2][k]);
+            fill_rec3<L0, L1, L2, K0, NV, EX2>(buf + lane * RB, (double)bl.c[0][i], (double)bl.c[1][j],
+                                               (double)bl.c[2][k], (double)bl.z[0][i], (double)bl.z[1][j],
+                                               (double)bl.z[2][k]);
         }
         __syncwarp();
+        int q = 0;
+        const char* rec = buf;
+        // the exponentials of kIlp triples in flight, then their multiply-adds
+        constexpr int kIlp = NV <= 6 ? 4 : 2;
 #pragma unroll 1
-        for (int q8 = 0; q8 < m; q8 += 8) {
-            const int qe = min(q8 + 8, m);
-            int q = q8;
-            const char* rec = buf + q8 * RB;
-            // the exponentials of kIlp triples in flight, then their multiply-adds
-            constexpr int kIlp = NV <= 6 ? 4 : 2;
-#pragma unroll 1
-            for (; q + kIlp <= qe; q += kIlp, rec += kIlp * RB) {
-                FT e[kIlp];
+        for (; q + kIlp <= m; q += kIlp, rec += kIlp * RB) {
+            double e[kIlp];
 #pragma unroll
-                for (int u = 0; u < kIlp; ++u) e[u] = rec_exp3(rec + u * RB, R0, R1, R2, FT(0));
+            for (int u = 0; u < kIlp; ++u) e[u] = rec_exp3<EX2>(rec + u * RB, R0, R1, R2);
 #pragma unroll
-                for (int u = 0; u < kIlp; ++u) add_rec3<NV>(rec + u * RB, e[u], part);
-            }
-#pragma unroll 1
-            for (; q < qe; ++q, rec += RB) add_rec3<NV>(rec, rec_exp3(rec, R0, R1, R2, FT(0)), part);
-            if constexpr (F32) {
-                if (qb == q0 && q8 == 0) {  // the first run opens the sums
-#pragma unroll
-                    for (int i = 0; i < NV; ++i) hi[i] = (i & 1) ? part[i / 2].y : part[i / 2].x;
-                } else {
-#pragma unroll
-                    for (int i = 0; i < NV; ++i) {
-                        float s, e;
-                        two_sum(hi[i], (i & 1) ? part[i / 2].y : part[i / 2].x, s, e);
-                        hi[i] = s;
-                        lo[i] += e;
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < NP; ++i) part[i] = Acc{};
-            }
+            for (int u = 0; u < kIlp; ++u) add_rec3<NV>(rec + u * RB, e[u], sum);
         }
-    }
-    if constexpr (!F32) {
-#pragma unroll
-        for (int i = 0; i < NV; ++i) hi[i] = part[i];
+#pragma unroll 1
+        for (; q < m; ++q, rec += RB) add_rec3<NV>(rec, rec_exp3<EX2>(rec, R0, R1, R2), sum);
     }
 }
 
 // The slots from K0 on, kMomSlots3 at a time, to row out[32 (slot)] (a column per lane).
 // split: the CTA's warps take a share of the triples each and their sums meet in xbuf, added
 // in warp order by warp 0.
-template <int L0, int L1, int L2, int K0, typename FT, typename IT>
-__device__ __forceinline__ void moments3_from(const Block3<IT>& bl, int n, char* buf, const double (&R)[3], FT* out,
-                                              bool split, FT* xbuf) {
+template <int L0, int L1, int L2, int K0, typename FT>
+__device__ __forceinline__ void moments3_from(const Block3<FT>& bl, int n, char* buf, const double (&R)[3], double* out,
+                                              bool split, double* xbuf) {
     constexpr int D = Prog3<L0, L1, L2, 0, 1>::D, NCH = (D + kMomSlots3 - 1) / kMomSlots3, S = (D + NCH - 1) / NCH;
     constexpr int NV = K0 + S <= D ? S : D - K0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int per = split ? (n + 8 * kWarps3 - 1) / (8 * kWarps3) * 8 : n;
     const int q0 = split ? min(n, warp * per) : 0, q1 = min(n, q0 + per);
-    FT hi[NV], lo[NV];
-    moments3<L0, L1, L2, K0, NV, FT>(bl, q0, q1, buf, R, hi, lo);
-    constexpr bool F32 = sizeof(FT) == 4;
+    double sum[NV];
+    moments3<L0, L1, L2, K0, NV, FT>(bl, q0, q1, buf, R, sum);
     if (split) {
         if (warp > 0) {
 #pragma unroll
-            for (int i = 0; i < NV; ++i) {
-                FT* x = xbuf + ((warp - 1) * kMomSlots3 + i) * (F32 ? 64 : 32) + lane;
-                x[0] = hi[i];
-                if constexpr (F32) x[32] = lo[i];
-            }
+            for (int i = 0; i < NV; ++i) xbuf[((warp - 1) * kMomSlots3 + i) * 32 + lane] = sum[i];
         }
         __syncthreads();
         if (warp == 0) {
 #pragma unroll 1
             for (int w = 0; w < kWarps3 - 1; ++w)
 #pragma unroll
-                for (int i = 0; i < NV; ++i) {
-                    const FT* x = xbuf + (w * kMomSlots3 + i) * (F32 ? 64 : 32) + lane;
-                    if constexpr (F32) {
-                        float s, e;
-                        two_sum(hi[i], x[0], s, e);
-                        hi[i] = s;
-                        lo[i] += x[32] + e;
-                    } else {
-                        hi[i] += x[0];
-                    }
-                }
+                for (int i = 0; i < NV; ++i) sum[i] += xbuf[(w * kMomSlots3 + i) * 32 + lane];
         }
         __syncthreads();  // xbuf is free for the next slots
     }
     if (!split || warp == 0) {
-        FT bad = FT(0);
-        if constexpr (F32) {  // NaN when a distance is infinite or NaN (see ex2_neg3)
-            const double all = R[0] + R[1] + R[2];
-            bad = __double2float_rn(all - all);
+        if constexpr (fast_exp3<FT>(L0)) {  // NaN when a distance is infinite or NaN (see ex2_neg3)
+            const double all = R[0] + R[1] + R[2], bad = all - all;
+#pragma unroll
+            for (int i = 0; i < NV; ++i) sum[i] += bad;
         }
 #pragma unroll
-        for (int i = 0; i < NV; ++i) out[32 * (K0 + i) + lane] = F32 ? (hi[i] + lo[i]) + bad : hi[i];
+        for (int i = 0; i < NV; ++i) out[32 * (K0 + i) + lane] = sum[i];
     }
     if constexpr (K0 + S < D) moments3_from<L0, L1, L2, K0 + S, FT>(bl, n, buf, R, out, split, xbuf);
 }
-template <int L0, int L1, int L2, typename FT, typename IT>
-__device__ __noinline__ void moments3_call(const Block3<IT>& bl, int n, char* buf, const double (&R)[3], FT* out,
-                                           bool split, FT* xbuf) {
+template <int L0, int L1, int L2, typename FT>
+__device__ __noinline__ void moments3_call(const Block3<FT>& bl, int n, char* buf, const double (&R)[3], double* out,
+                                           bool split, double* xbuf) {
     moments3_from<L0, L1, L2, 0, FT>(bl, n, buf, R, out, split, xbuf);
 }
 
@@ -436,38 +369,37 @@ struct Dest3 {
     bool on;         // the lane's element is in this pass
 };
 template <int L0, int L1, int L2, int PART, int NP, typename FT>
-__device__ __forceinline__ void transform3_slab(const FT* mom, const Geo3<FT>& g, int o0, int o1, int o2,
+__device__ __forceinline__ void transform3_slab(const double* mom, const Geo3<FT>& g, int o0, int o1, int o2,
                                                 const Dest3<FT>& to) {
     const int lane = threadIdx.x & 31;
-    using AT = std::conditional_t<(L0 > 2), double, FT>;  // see mom_words3
-    const AT* m = reinterpret_cast<const AT*>(mom) + lane;
-    AT d01[3], d02[3], d12[3];
+    const double* m = mom + lane;
+    double d01[3], d02[3], d12[3];
     if constexpr (L0 > 0) {
-        const AT s01 = o0 < o1 ? AT(1) : AT(-1), s02 = o0 < o2 ? AT(1) : AT(-1), s12 = o1 < o2 ? AT(1) : AT(-1);
+        const double s01 = o0 < o1 ? 1.0 : -1.0, s02 = o0 < o2 ? 1.0 : -1.0, s12 = o1 < o2 ? 1.0 : -1.0;
         const int p01 = 3 * pair3(o0, o1), p02 = 3 * pair3(o0, o2), p12 = 3 * pair3(o1, o2);
 #pragma unroll
         for (int x = 0; x < 3; ++x) {
-            d01[x] = s01 * (AT)g.d[p01 + x][lane];
-            d02[x] = s02 * (AT)g.d[p02 + x][lane];
-            d12[x] = s12 * (AT)g.d[p12 + x][lane];
+            d01[x] = s01 * g.d[p01 + x][lane];
+            d02[x] = s02 * g.d[p02 + x][lane];
+            d12[x] = s12 * g.d[p12 + x][lane];
         }
     }
     FT* row = to.row;
     const int t0 = to.t0, t1 = to.t1, t2 = to.t2;
     const bool on = to.on;
-    transform3<L0, L1, L2, PART, NP, AT>([&](int k) { return __ldcs(m + 32 * k); }, d01, d02, d12,
-                                         [&](int c0, int c1, int c2, AT v) {
-                                             if (on) row[c0 * t0 + c1 * t1 + c2 * t2] = (FT)v;
-                                         });
+    transform3<L0, L1, L2, PART, NP, double>([&](int k) { return __ldcs(m + 32 * k); }, d01, d02, d12,
+                                             [&](int c0, int c1, int c2, double v) {
+                                                 if (on) row[c0 * t0 + c1 * t1 + c2 * t2] = (FT)v;
+                                             });
 }
 template <int L0, int L1, int L2, int PART, int NP, typename FT>
-__device__ __noinline__ void transform3_call(const FT* mom, const Geo3<FT>& g, int o0, int o1, int o2,
+__device__ __noinline__ void transform3_call(const double* mom, const Geo3<FT>& g, int o0, int o1, int o2,
                                              const Dest3<FT>& to) {
     transform3_slab<L0, L1, L2, PART, NP, FT>(mom, g, o0, o1, o2, to);
 }
 
 template <int L0, int L1, int L2, int NP, typename FT>
-__device__ __forceinline__ void block3_part(int part, const FT* mom, const Geo3<FT>& g, int o0, int o1, int o2,
+__device__ __forceinline__ void block3_part(int part, const double* mom, const Geo3<FT>& g, int o0, int o1, int o2,
                                             const Dest3<FT>& to) {
     if constexpr (L0 + L1 + L2 <= 2) {
         transform3_slab<L0, L1, L2, 0, 1, FT>(mom, g, o0, o1, o2, to);
@@ -509,7 +441,7 @@ struct Ov3Params {
     const int* segs;     // segment starts in items (nseg + 1 entries); nseg, H, pick at segs[nitems + 1], [nitems + 2], [nitems + 3]
     const Panel3* panels;
     const Out3* table;   // the panels' output elements
-    FT* mom;             // moments of tile t: mom + (t - tile0) * slots * 32
+    double* mom;         // moments of tile t: mom + (t - tile0) * slots * 32
     int tile0, round;    // this launch's tiles: [tile0, tile0 + round)
     int nitems, npanels, slots, ns, K, N, NZ;
     FT scale;
@@ -526,7 +458,7 @@ template <typename FT>
 __global__ void __launch_bounds__(kThreads3, kMomCtas3) k_moments3(const __grid_constant__ Ov3Params<FT> P) {
     constexpr int W = kWarps3;
     __shared__ __align__(16) char recbuf[W][kRecBytes3];
-    __shared__ __align__(16) FT xbuf[(W - 1) * kMomSlots3 * (sizeof(FT) == 4 ? 64 : 32)];
+    __shared__ __align__(16) double xbuf[(W - 1) * kMomSlots3 * 32];
     __shared__ unsigned claim;
     pdl_wait();  // launched programmatically after k_overlap3c or the last round: the bins, the prep's order and the
                  // buffers are complete past here
@@ -580,16 +512,14 @@ __global__ void __launch_bounds__(kThreads3, kMomCtas3) k_moments3(const __grid_
             }
             const int n = bl.n[0] * bl.n[1] * bl.n[2];
             if (n == 0) continue;  // k_transform3 writes zeros
-            FT* out = P.mom + ((size_t)tile * P.slots + wi.moff) * 32;
+            double* out = P.mom + ((size_t)tile * P.slots + wi.moff) * 32;
             switch (wi.cls) {
-#define AOK_X(a, b, c, np)                                                                 \
-    case class3(a, b, c):                                                                  \
-        if constexpr (a + b + c <= 2)                                                      \
-            moments3_from<a, b, c, 0, FT>(bl, n, recbuf[warp], R, out, split, xbuf);       \
-        else if constexpr (a <= 2)                                                         \
-            moments3_call<a, b, c, FT>(bl, n, recbuf[warp], R, out, split, xbuf);          \
-        else                                                                               \
-            moments3_call<a, b, c, double>(bl, n, recbuf[warp], R, (double*)out, split, (double*)xbuf); \
+#define AOK_X(a, b, c, np)                                                           \
+    case class3(a, b, c):                                                            \
+        if constexpr (a + b + c <= 2)                                                \
+            moments3_from<a, b, c, 0, FT>(bl, n, recbuf[warp], R, out, split, xbuf); \
+        else                                                                         \
+            moments3_call<a, b, c, FT>(bl, n, recbuf[warp], R, out, split, xbuf);    \
         break;
                 AOK_CLASSES3(AOK_X)
                 default: break;
@@ -609,7 +539,7 @@ struct Unit3 {
 };
 
 template <typename FT>
-__global__ void __launch_bounds__(kTrThreads3<FT>, kTrCtas3<FT>) k_transform3(const __grid_constant__ Ov3Params<FT> P) {
+__global__ void __launch_bounds__(kTrThreads3, 1) k_transform3(const __grid_constant__ Ov3Params<FT> P) {
     extern __shared__ __align__(16) char smem[];
     __shared__ Unit3 units[2];
     __shared__ unsigned s_u[2];
@@ -637,10 +567,9 @@ __global__ void __launch_bounds__(kTrThreads3<FT>, kTrCtas3<FT>) k_transform3(co
         const int key = td.x, ga = key / (P.NZ * P.NZ), gb = (key / P.NZ) % P.NZ, gc = key % P.NZ;
         const bool on = lane < pn.nsa;
         const int sa = pn.sa0 + (on ? lane : 0), la = P.l[sa], lb = P.l[pn.sb], lc = P.l[pn.sc];
-        const int cls = canon3(la, lb, lc).cls;
-        const ClassInfo3 ci = kClass3[cls];
+        const ClassInfo3 ci = kClass3[canon3(la, lb, lc).cls];
         const bool zero = P.pn[ga * P.ns + sa] * P.pn[gb * P.ns + pn.sb] * P.pn[gc * P.ns + pn.sc] == 0;
-        const int t0 = on ? (zero ? 1 : ci.parts) : 0, s0 = on ? ncart(la) * ncart(lb) * ncart(lc) : 0, m0 = on ? ci.D * mom_words3<FT>(cls) : 0;
+        const int t0 = on ? (zero ? 1 : ci.parts) : 0, s0 = on ? ncart(la) * ncart(lb) * ncart(lc) : 0, m0 = on ? ci.D : 0;
         int t = t0, so = s0, m = m0;
 #pragma unroll
         for (int o = 1; o < kPanelItems3; o <<= 1) {
@@ -682,12 +611,12 @@ __global__ void __launch_bounds__(kTrThreads3<FT>, kTrCtas3<FT>) k_transform3(co
         __syncthreads();  // the unit is set up, the slab is free
         const Unit3& U = units[f];
         if (U.tile < 0) break;
-        if (threadIdx.x == kTrThreads3<FT> - 1) s_u[f] = atomicAdd(P.counter + 1, 1u);  // the next unit
+        if (threadIdx.x == kTrThreads3 - 1) s_u[f] = atomicAdd(P.counter + 1, 1u);  // the next unit
         const Panel3 pn = U.pn;
         const int lb = P.l[pn.sb], lc = P.l[pn.sc], NB = ncart(lb), NC = ncart(lc);
         const int lanes = 32 / pn.passes, rowlen = (pn.comps + 1) | 1;
         const int nt = pn.pass * lanes < U.cnt ? U.t[pn.nsa] : 0;  // a partial tile may not reach this pass
-        const FT* tile_mom = P.mom + (size_t)U.tile * P.slots * 32;
+        const double* tile_mom = P.mom + (size_t)U.tile * P.slots * 32;
         FT* row = slab + (size_t)(lane & (lanes - 1)) * rowlen;
         if (warp == 0 && lane < lanes) row[pn.comps] = FT(0);
         for (;;) {
@@ -711,7 +640,7 @@ __global__ void __launch_bounds__(kTrThreads3<FT>, kTrCtas3<FT>) k_transform3(co
             to.t0 = cn.o0 == 0 ? 1 : cn.o0 == 1 ? sj : sk;
             to.t1 = cn.o1 == 0 ? 1 : cn.o1 == 1 ? sj : sk;
             to.t2 = cn.o2 == 0 ? 1 : cn.o2 == 1 ? sj : sk;
-            const FT* mom = tile_mom + (size_t)U.moff[i] * 32;
+            const double* mom = tile_mom + (size_t)U.moff[i] * 32;
             switch (cn.cls) {
 #define AOK_X(a, b, c, np) \
     case class3(a, b, c): block3_part<a, b, c, np, FT>(part, mom, geo[f], cn.o0, cn.o1, cn.o2, to); break;
@@ -721,13 +650,13 @@ __global__ void __launch_bounds__(kTrThreads3<FT>, kTrCtas3<FT>) k_transform3(co
             }
         }
         __syncthreads();
-        if (warp == kTrThreads3<FT> / 32 - 1) fetch(f ^ 1, s_u[f]);
+        if (warp == kTrThreads3 / 32 - 1) fetch(f ^ 1, s_u[f]);
         // the slab streams out
         const int e0 = pn.pass * lanes, ne = min(lanes, U.cnt - e0);
         FT* out = P.out + (size_t)P.boff[pn.sc] * N2 + (size_t)P.boff[pn.sb] * P.N + P.boff[pn.sa0];
         const long long* at = geo[f].at + e0;
 #pragma unroll 1
-        for (int x0 = 32 * warp; x0 < pn.nout; x0 += kTrThreads3<FT>) {
+        for (int x0 = 32 * warp; x0 < pn.nout; x0 += kTrThreads3) {
             const int x = x0 + lane;
             const bool in = x < pn.nout;
             const Out3 q = P.table[pn.tab + (in ? x : 0)];
@@ -773,7 +702,7 @@ inline int launch_moments3(aok_plan* p, void* out, const void* posA, const void*
     P.segs = p->d_segsm;
     P.panels = (const Panel3*)p->d_panels3;
     P.table = (const Out3*)p->d_out3;
-    P.mom = (FT*)p->d_mom3;
+    P.mom = (double*)p->d_mom3;
     P.round = p->round3;
     P.nitems = p->nitemsm;
     P.npanels = p->npanels3;
@@ -790,7 +719,7 @@ inline int launch_moments3(aok_plan* p, void* out, const void* posA, const void*
     auto tr = k_transform3<FT>;
     int st;
     if ((st = kernel_prepare((const void*)mom, 0, kThreads3, nullptr)) != AOK_OK) return st;
-    if ((st = kernel_prepare((const void*)tr, kTrSmem3<FT>, kTrThreads3<FT>, nullptr)) != AOK_OK) return st;
+    if ((st = kernel_prepare((const void*)tr, kTrSmem3, kTrThreads3, nullptr)) != AOK_OK) return st;
     // a tile per 32 elements and one partial tile per species triple
     const int64_t most = (B + 31) / 32 + p->NZ * p->NZ * p->NZ;
     const int rounds = (int)((most + p->round3 - 1) / p->round3);
@@ -799,7 +728,7 @@ inline int launch_moments3(aok_plan* p, void* out, const void* posA, const void*
         P.tile0 = r * p->round3;
         P.counter = p->d_cnt3 + 2 * r;
         e = launch_pdl(mom, dim3(p->num_sms * kMomCtas3), dim3(kThreads3), 0, s, P);
-        if (e == cudaSuccess) e = launch_pdl(tr, dim3(p->num_sms * kTrCtas3<FT>), dim3(kTrThreads3<FT>), kTrSmem3<FT>, s, P);
+        if (e == cudaSuccess) e = launch_pdl(tr, dim3(p->num_sms), dim3(kTrThreads3), kTrSmem3, s, P);
     }
     timing_end(p, s);  // begun before the explicit tables' kernel (launch_ov3)
     return cuda_status(e, "k_transform3");
