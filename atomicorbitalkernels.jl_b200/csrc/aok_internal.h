@@ -70,15 +70,16 @@ struct aok_plan {
     void* d_order3 = nullptr;        // per call: the items in queue order (k_prep3c)
     int* d_segs3 = nullptr;          // per call: segment starts in d_order3 (nitems3 + 1), then the count
     int* d_key3 = nullptr;           // what d_order3/d_segs3 were built from: (n, tiles, target, counts)
-    // contracted bases with f shells (overlap3c_moments.cu): items, order, segments and their
-    // key as above, panels and moments
-    void* d_itemsm = nullptr;
+    // contracted bases with f shells (overlap3c_moments.cu): moments, and one buffer with the
+    // schedule: items, order, segments and their key as above, panels, counters
+    void* d_mom3 = nullptr;          // moments of round3 tiles: slots3 x 32 each; set when all of this is
+    void* d_sched3 = nullptr;
+    void* d_itemsm = nullptr;        // in d_sched3, as the following
     void* d_orderm = nullptr;
     int* d_segsm = nullptr;
     int* d_keym = nullptr;
     void* d_panels3 = nullptr;
     void* d_out3 = nullptr;          // the panels' output elements
-    void* d_mom3 = nullptr;          // moments of round3 tiles: slots3 x 32 each
     unsigned* d_cnt3 = nullptr;      // two work counters per round
     int nitems3 = 0, nitemsm = 0, npanels3 = 0, slots3 = 0, round3 = 0, nrounds3 = 0;
     // graph mode of the fixed-basis forward (aok_plan_set_graph): the instantiated

@@ -56,6 +56,7 @@ int set_error(int code, const std::string& msg) {
 
 int cuda_status(cudaError_t e, const char* what) {
     if (e == cudaSuccess) return AOK_OK;
+    (void)cudaGetLastError();  // a later launch's check shall not find this error again
     return set_error(AOK_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
@@ -181,8 +182,7 @@ int aok_plan_destroy(aok_plan* p) {
                     p->d_items,     p->d_blockhist, p->d_gb_zeta,    p->d_gb_coef,
                     p->d_pb_rec,    p->d_pb_counts, p->d_pb_items,  p->d_pb_itemidx, p->d_pb_rows,
                     p->d_partials,  p->d_coef_scratch, p->d_pp3,    p->d_npp3,       p->d_items3,    p->d_order3,    p->d_segs3,     p->d_key3,
-                    p->d_itemsm,    p->d_orderm,    p->d_segsm,     p->d_keym,
-                    p->d_panels3,   p->d_out3,      p->d_mom3,      p->d_cnt3,
+                    p->d_sched3,    p->d_mom3,
                     p->d_pk,        p->d_segs,      p->d_nseg,      p->d_dpos_rec,   p->d_dpos_counts,
                     p->d_dpos_items};
     for (void* b : bufs) dfree(b);

@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(kOrder3Threads) k_prep3c(FT* __restrict__ pz, 
 static bool may_moments3(const aok_plan* p) { return p->Lmax > kMaxL3Spec && p->K > 1; }
 
 int setup_overlap3c_schedule(aok_plan* p) {
-    if (p->d_key3 && (p->d_panels3 || !may_moments3(p))) return AOK_OK;
+    if (p->d_key3) return may_moments3(p) ? m3::setup_moments3(p) : AOK_OK;
     if (p->NZ * p->NZ * p->NZ > kMaxPairs)
         return set_error(AOK_ERR_UNSUPPORTED, "3C overlap: more than 6 species (NZ^3 > 256 species triples)");
     if (p->Lmax > kMaxL3) return set_error(AOK_ERR_UNSUPPORTED, "3C overlap: shells above l = 3");
@@ -308,27 +308,40 @@ int setup_overlap3c_schedule(aok_plan* p) {
     for (auto& x : v) items.push_back(x.second);
     p->nitems3 = (int)items.size();
     const size_t fsz = p->prec == AOK_PREC_F64 ? sizeof(double) : sizeof(float);
+    // after a failure the plan has none of these buffers, and the next call starts again
+    auto drop = [](auto*& b) {
+        if (b) cudaFree(b);
+        b = nullptr;
+    };
+    auto fail = [&](cudaError_t e, const char* what) {
+        drop(p->d_items3);
+        drop(p->d_order3);
+        drop(p->d_segs3);
+        drop(p->d_pp3);
+        drop(p->d_npp3);
+        drop(p->d_key3);
+        return cuda_status(e, what);
+    };
     cudaError_t e;
     if ((e = cudaMalloc(&p->d_items3, sizeof(Item3) * items.size())) != cudaSuccess)
-        return cuda_status(e, "cudaMalloc(items3)");
+        return fail(e, "cudaMalloc(items3)");
     if ((e = cudaMalloc(&p->d_order3, sizeof(Item3) * items.size())) != cudaSuccess)
-        return cuda_status(e, "cudaMalloc(order3)");
+        return fail(e, "cudaMalloc(order3)");
     if ((e = cudaMalloc(&p->d_segs3, sizeof(int) * (items.size() + 3))) != cudaSuccess)
-        return cuda_status(e, "cudaMalloc(segs3)");
+        return fail(e, "cudaMalloc(segs3)");
     if ((e = cudaMemcpy(p->d_items3, items.data(), sizeof(Item3) * items.size(), cudaMemcpyHostToDevice)) !=
         cudaSuccess)
-        return cuda_status(e, "cudaMemcpy(items3)");
+        return fail(e, "cudaMemcpy(items3)");
     // compact primitive lists: zeta then coef, each ns*K*NZ, and the ns*NZ lengths
     if ((e = cudaMalloc(&p->d_pp3, 2 * fsz * (size_t)(ns * p->K * p->NZ))) != cudaSuccess)
-        return cuda_status(e, "cudaMalloc(prim3)");
+        return fail(e, "cudaMalloc(prim3)");
     if ((e = cudaMalloc(&p->d_npp3, sizeof(int) * (size_t)(ns * p->NZ))) != cudaSuccess)
-        return cuda_status(e, "cudaMalloc(nprim3)");
+        return fail(e, "cudaMalloc(nprim3)");
     // the schedule key of k_prep3c: all ones (n = -1) matches no call, so the first builds
     const size_t kbytes = sizeof(int) * (size_t)(4 + ns * p->NZ);
-    if ((e = cudaMalloc(&p->d_key3, kbytes)) != cudaSuccess) return cuda_status(e, "cudaMalloc(key3)");
-    if ((e = cudaMemset(p->d_key3, 0xFF, kbytes)) != cudaSuccess) return cuda_status(e, "cudaMemset(key3)");
-    if (may_moments3(p)) return m3::setup_moments3(p);
-    return AOK_OK;
+    if ((e = cudaMalloc(&p->d_key3, kbytes)) != cudaSuccess) return fail(e, "cudaMalloc(key3)");
+    if ((e = cudaMemset(p->d_key3, 0xFF, kbytes)) != cudaSuccess) return fail(e, "cudaMemset(key3)");
+    return may_moments3(p) ? m3::setup_moments3(p) : AOK_OK;
 }
 
 // The kernel's unit counter (32 bits, each warp claims one past the end) must not

@@ -232,7 +232,7 @@ static int panel_table3(const aok_plan* p, const Panel3& pn, std::vector<Out3>* 
 }
 
 int setup_moments3(aok_plan* p) {
-    if (p->d_panels3) return AOK_OK;
+    if (p->d_mom3) return AOK_OK;
     const int ns = (int)p->ns;
     const size_t fsz = p->prec == AOK_PREC_F64 ? sizeof(double) : sizeof(float);
     // Panels: per (B shell, C shell), runs of A shells whose blocks fit the CTA's slab; a
@@ -293,41 +293,53 @@ int setup_moments3(aok_plan* p) {
     std::stable_sort(items.begin(), items.end(), [](const Item3& a, const Item3& b) { return a.cls > b.cls; });
     p->nitemsm = (int)items.size();
     p->slots3 = slots;
-    // moments are kept for at most kMoments3 bytes of tiles at a time (in the L2 cache); a
-    // larger batch goes through in rounds.  One tile always fits: the panel schedule of the
-    // plan bounds N to about 120 (64 shells of 83 functions, FP64: 70 MB).
-    const int64_t most = (p->max_batch + 31) / 32 + bin_keys_max(p->NZ) + 1, tile = (int64_t)slots * 32 * (int64_t)sizeof(double);
+    // moments are kept for at most kMoments3 bytes of tiles at a time; a larger batch goes
+    // through in rounds.  One tile always fits: the panel schedule of the plan bounds N to
+    // about 120 (64 shells of 83 functions: 70 MB).
+    const int64_t most = (p->max_batch + 31) / 32 + bin_keys_max(p->NZ) + 1;
+    const int64_t tile = (int64_t)slots * 32 * (int64_t)sizeof(double);
     p->round3 = (int)std::max<int64_t>(1, std::min(most, kMoments3 / tile));
     p->nrounds3 = (int)((most + p->round3 - 1) / p->round3);
     p->npanels3 = (int)panels.size();
-    cudaError_t e;
-    void* d = nullptr;
-    if ((e = cudaMalloc(&p->d_itemsm, sizeof(Item3) * items.size())) != cudaSuccess)
-        return cuda_status(e, "cudaMalloc(items3)");
-    if ((e = cudaMalloc(&p->d_orderm, sizeof(Item3) * items.size())) != cudaSuccess)
-        return cuda_status(e, "cudaMalloc(order3)");
-    if ((e = cudaMalloc(&p->d_segsm, sizeof(int) * (items.size() + 4))) != cudaSuccess)
-        return cuda_status(e, "cudaMalloc(segs3)");
-    if ((e = cudaMemcpy(p->d_itemsm, items.data(), sizeof(Item3) * items.size(), cudaMemcpyHostToDevice)) !=
-        cudaSuccess)
-        return cuda_status(e, "cudaMemcpy(items3)");
-    if ((e = cudaMalloc(&p->d_mom3, (size_t)(tile * p->round3))) != cudaSuccess)
-        return cuda_status(e, "cudaMalloc(moments3)");
-    if ((e = cudaMalloc(&p->d_cnt3, sizeof(unsigned) * 2 * (size_t)p->nrounds3)) != cudaSuccess)
-        return cuda_status(e, "cudaMalloc(counters3)");
-    // the schedule key of k_prepm3: all ones (n = -1) matches no call, so the first builds
-    const size_t kbytes = sizeof(int) * (size_t)(4 + ns * p->NZ);
-    if ((e = cudaMalloc(&p->d_keym, kbytes)) != cudaSuccess) return cuda_status(e, "cudaMalloc(key3)");
-    if ((e = cudaMemset(p->d_keym, 0xFF, kbytes)) != cudaSuccess) return cuda_status(e, "cudaMemset(key3)");
-    if ((e = cudaMalloc(&p->d_out3, sizeof(Out3) * table.size())) != cudaSuccess)
-        return cuda_status(e, "cudaMalloc(out3)");
-    if ((e = cudaMemcpy(p->d_out3, table.data(), sizeof(Out3) * table.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
-        return cuda_status(e, "cudaMemcpy(out3)");
-    if ((e = cudaMalloc(&d, sizeof(Panel3) * panels.size())) != cudaSuccess)
-        return cuda_status(e, "cudaMalloc(panels3)");
-    p->d_panels3 = d;
-    e = cudaMemcpy(d, panels.data(), sizeof(Panel3) * panels.size(), cudaMemcpyHostToDevice);
-    return cuda_status(e, "cudaMemcpy(panels3)");
+    // one buffer: items, panels, output elements and the schedule key of k_prepm3 (all ones:
+    // n = -1 matches no call, so the first builds), copied in one piece; then what the
+    // kernels write
+    size_t bytes = 0;
+    auto place = [&](size_t n) {
+        const size_t at = bytes;
+        bytes += (n + 255) / 256 * 256;
+        return at;
+    };
+    const size_t nitems = sizeof(Item3) * items.size(), npanels = sizeof(Panel3) * panels.size(),
+                 nout = sizeof(Out3) * table.size(), nkey = sizeof(int) * (size_t)(4 + ns * p->NZ);
+    const size_t at_items = place(nitems), at_panels = place(npanels), at_out = place(nout), at_key = place(nkey);
+    std::vector<char> host(bytes);
+    memcpy(host.data() + at_items, items.data(), nitems);
+    memcpy(host.data() + at_panels, panels.data(), npanels);
+    memcpy(host.data() + at_out, table.data(), nout);
+    memset(host.data() + at_key, 0xFF, nkey);
+    const size_t at_order = place(nitems), at_segs = place(sizeof(int) * (items.size() + 4)),
+                 at_cnt = place(sizeof(unsigned) * 2 * (size_t)p->nrounds3);
+    // on a failure the plan has neither buffer, and the next call starts again
+    void *sched = nullptr, *mom = nullptr;
+    cudaError_t e = cudaMalloc(&sched, bytes);
+    if (e == cudaSuccess) e = cudaMemcpy(sched, host.data(), host.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMalloc(&mom, (size_t)(tile * p->round3));
+    if (e != cudaSuccess) {
+        if (sched) cudaFree(sched);
+        return cuda_status(e, "3C overlap: moments");
+    }
+    char* base = (char*)sched;
+    p->d_sched3 = sched;
+    p->d_itemsm = base + at_items;
+    p->d_panels3 = base + at_panels;
+    p->d_out3 = base + at_out;
+    p->d_keym = (int*)(base + at_key);
+    p->d_orderm = base + at_order;
+    p->d_segsm = (int*)(base + at_segs);
+    p->d_cnt3 = (unsigned*)(base + at_cnt);
+    p->d_mom3 = mom;
+    return AOK_OK;
 }
 
 // The prep of the moment path on stream `side`, after k_prep3c (see k_prepm3).
