@@ -73,6 +73,7 @@ struct aok_plan {
     // contracted bases with f shells (overlap3c_moments.cu): moments, and one buffer with the
     // schedule: items, order, segments and their key as above, panels, counters
     void* d_mom3 = nullptr;          // moments of round3 tiles: slots3 x 32 each; set when all of this is
+    bool no_mom3 = false;            // there was no memory for it: explicit tables for this plan
     void* d_sched3 = nullptr;
     void* d_itemsm = nullptr;        // in d_sched3, as the following
     void* d_orderm = nullptr;

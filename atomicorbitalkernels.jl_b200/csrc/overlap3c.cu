@@ -278,7 +278,8 @@ __global__ void __launch_bounds__(kOrder3Threads) k_prep3c(FT* __restrict__ pz, 
 // from the counts per shell), the others go through explicit E tables.  Up to d the tables
 // win for common bases (15 functions, FP32C: 19 against 32 us for 100 elements, 117 against
 // 141 for 4,096), and with one primitive per shell (FP32C 94 against 141 us for 33 elements,
-// 184 against 226 for 400, 421 against 375 for 900).
+// 184 against 226 for 400, 421 against 375 for 900).  A plan without memory for the moments
+// has the tables alone (setup_moments3).
 static bool may_moments3(const aok_plan* p) { return p->Lmax > kMaxL3Spec && p->K > 1; }
 
 int setup_overlap3c_schedule(aok_plan* p) {
@@ -388,7 +389,7 @@ template <typename Bin>
 static int launch_overlap3c(aok_plan* p, void* out, const void* zeta, const void* coef, const int64_t* nprim,
                             const int64_t* prim_offset, const void* posA, const void* posB, const void* posC,
                             int64_t B, double lengthscale, cudaStream_t s, Bin bin, bool chain) {
-    const bool moments = may_moments3(p);
+    const bool moments = p->d_mom3 != nullptr;
     auto prep = [&](cudaStream_t on, bool pdl) {
         const int st = launch_prep3c(p, zeta, coef, nprim, prim_offset, B, on, pdl);
         if (st != AOK_OK || !moments) return st;

@@ -232,7 +232,7 @@ static int panel_table3(const aok_plan* p, const Panel3& pn, std::vector<Out3>* 
 }
 
 int setup_moments3(aok_plan* p) {
-    if (p->d_mom3) return AOK_OK;
+    if (p->d_mom3 || p->no_mom3) return AOK_OK;
     const int ns = (int)p->ns;
     const size_t fsz = p->prec == AOK_PREC_F64 ? sizeof(double) : sizeof(float);
     // Panels: per (B shell, C shell), runs of A shells whose blocks fit the CTA's slab; a
@@ -320,14 +320,18 @@ int setup_moments3(aok_plan* p) {
     memset(host.data() + at_key, 0xFF, nkey);
     const size_t at_order = place(nitems), at_segs = place(sizeof(int) * (items.size() + 4)),
                  at_cnt = place(sizeof(unsigned) * 2 * (size_t)p->nrounds3);
-    // on a failure the plan has neither buffer, and the next call starts again
+    // on a failure the plan has neither buffer; without memory it keeps to the explicit tables,
+    // which need none of this (for good: a later call may be under stream capture, where
+    // nothing can be allocated), after another failure the next call starts again
     void *sched = nullptr, *mom = nullptr;
     cudaError_t e = cudaMalloc(&sched, bytes);
     if (e == cudaSuccess) e = cudaMemcpy(sched, host.data(), host.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMalloc(&mom, (size_t)(tile * p->round3));
     if (e != cudaSuccess) {
         if (sched) cudaFree(sched);
-        return cuda_status(e, "3C overlap: moments");
+        const int st = cuda_status(e, "3C overlap: moments");
+        p->no_mom3 = e == cudaErrorMemoryAllocation;
+        return p->no_mom3 ? AOK_OK : st;
     }
     char* base = (char*)sched;
     p->d_sched3 = sched;

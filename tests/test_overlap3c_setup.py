@@ -41,4 +41,35 @@ def test_failed_allocation_leaves_nothing_behind(tmp_path):
     for c in r["out"]:
         if c["failed"]:
             assert not c["got"], c                 # nothing launched
-        assert c["again"] == 0 and c["kept"] == 0 and c["same"], c
+            assert c["again"] == 0 and c["kept"] == 0 and c["same"], c
+
+
+NO_ROOM = """
+out = []
+for prec in (0, 1):
+    for gb in (False, True):
+        h = plan([0, 1, 2, 3], 3, 1 if gb else 2, prec, 5000)
+        base = fake.fake_live()
+        fake.fake_fail(-1, 1 << 20)                # the moments want more than that
+        for repeat in range(2):
+            ops()
+            if gb:
+                st = L.aok_overlap3c_gb(h, *[P(A)] * 8, I64(5000), P(0x77))
+            else:
+                st = L.aok_overlap3c(h, *[P(A)] * 9, I64(5000), F64(1.0), P(0x77))
+            out.append(dict(st=st, k=[k[0] for k in ops() if k[0].startswith("launch:")],
+                            n=fake.fake_live() - base))
+        fake.fake_fail(*NEVER)
+        L.aok_plan_destroy(h)
+print(json.dumps(dict(out=out, live=fake.fake_live(), bad=fake.fake_bad_frees())))
+"""
+
+
+def test_without_room_for_moments_the_tables_serve(tmp_path):
+    r = fakecuda.run(NO_ROOM, tmp_path)
+    assert r["live"] == 0 and r["bad"] == 0
+    assert len(r["out"]) == 8 and len({c["n"] for c in r["out"]}) == 1
+    for c in r["out"]:
+        assert c["st"] == 0, c
+        assert sum("k_overlap3c" in k for k in c["k"]) == 1
+        assert not any("moments3" in k or "transform3" in k or "prepm3" in k for k in c["k"]), c
