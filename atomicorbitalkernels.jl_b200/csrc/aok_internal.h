@@ -57,7 +57,8 @@ struct aok_plan {
     void* d_pb_rows = nullptr;       // per (species pair, item): unit sums (FP64, 4*K)
     void* d_partials = nullptr;      // per-CTA item sums
     int max_blocks = 0;
-    void* d_coef_scratch = nullptr;  // ns*K*NZ
+    void* d_coef_scratch = nullptr;  // compiled coefficients: two tables of ns*K*NZ (see aok_overlap2c_rrule)
+    void* rcoef = nullptr;           // the one that the last rrule forward wrote
     // position pullback (overlap2c_dpos.cu): records per (species pair, shell pair), their
     // counts, and the shell-pair list heaviest class first
     void* d_dpos_rec = nullptr;

@@ -158,7 +158,7 @@ int aok_plan_create(aok_plan** plan, int64_t nshells, const int64_t* ls, int64_t
         (st = dmalloc(&p->d_err, 1, "cudaMalloc(err)")) ||
         (st = dmalloc_bytes(&p->d_gb_zeta, (size_t)(nshells * K) * fsz, "cudaMalloc(gb_zeta)")) ||
         (st = dmalloc_bytes(&p->d_gb_coef, (size_t)(nshells * K) * fsz, "cudaMalloc(gb_coef)")) ||
-        (st = dmalloc_bytes(&p->d_coef_scratch, (size_t)(nshells * K * NZ) * fsz, "cudaMalloc(coef)")))
+        (st = dmalloc_bytes(&p->d_coef_scratch, 2 * (size_t)(nshells * K * NZ) * fsz, "cudaMalloc(coef)")))
         return fail(st);
     if ((st = cuda_status(cudaMemcpy(p->d_ls, ls32.data(), sizeof(int) * nshells, cudaMemcpyHostToDevice),
                           "cudaMemcpy(ls)")) ||
@@ -515,7 +515,14 @@ int aok_overlap2c_rrule(aok_plan* p, void* out, const void* zeta, const void* D,
     if (!p->ev_pb)
         AOK_TRY(cuda_status(cudaEventCreateWithFlags(&p->ev_pb, cudaEventDisableTiming), "cudaEventCreate"));
     p->basis_set = false;
+    // The pullback records of the last rrule forward may still be read from its coefficients on
+    // the side stream (only a pullback waits for them), so forwards take the two tables in
+    // turn: this stream waited for the side stream in that forward, which puts the records of
+    // the one before, from this table, in the past.
     void* coef = p->d_coef_scratch;
+    if (p->rcoef == coef)
+        coef = (char*)coef + (size_t)(p->ns * p->K * p->NZ) * (p->prec == AOK_PREC_F64 ? sizeof(double) : sizeof(float));
+    p->rcoef = coef;
     // this stream: coef, the forward records and the overlap kernel, the longest chain; side
     // stream: the bins, then the pullback records, beside the packing.  (The overlap kernel's
     // CTAs hold every register, so records prepared after the packing kept it from starting.)

@@ -106,9 +106,9 @@ int launch_pb_prepared(aok_plan* p, void* out0, void* out1, const void* dS, cons
                        cudaStream_t s) {
     AOK_TRY_PB(cuda_status(cudaStreamWaitEvent(s, p->ev_pb, 0), "cudaStreamWaitEvent"));
     if (p->prec == AOK_PREC_F64)
-        return launch_pb_f64(p, out0, out1, dS, dS2, alpha, zeta, p->d_coef_scratch, D, posA, posB, lengthscale,
+        return launch_pb_f64(p, out0, out1, dS, dS2, alpha, zeta, p->rcoef, D, posA, posB, lengthscale,
                              s, p->d_counter + 1);
-    return launch_pb_f32(p, out0, out1, dS, dS2, alpha, zeta, p->d_coef_scratch, D, posA, posB, lengthscale, s,
+    return launch_pb_f32(p, out0, out1, dS, dS2, alpha, zeta, p->rcoef, D, posA, posB, lengthscale, s,
                          p->d_counter + 1);
 }
 

@@ -36,8 +36,12 @@ static void op(const char* what, const void* a, const void* b) {
     snprintf(t, sizeof(t), "%s %lx %lx\n", what, (unsigned long)(uintptr_t)a, (unsigned long)(uintptr_t)b);
     ops += t;
 }
-static err_t launch(const void* f, stream_t s) {
-    op((names.count(f) ? "launch:" + names[f] : std::string("launch:?")).c_str(), s, 0);
+static err_t launch(const void* f, stream_t s, void** args) {
+    const std::string name = names.count(f) ? names[f] : "?";
+    // the coefficient table that the kernel writes (first argument) or reads (fourth)
+    const int coef = name.find("k_compile_coefI") != std::string::npos ? 0
+                     : name.find("k_prep_pbI") != std::string::npos    ? 3 : -1;
+    op(("launch:" + name).c_str(), s, coef < 0 ? 0 : *(void**)args[coef]);
     return 0;
 }
 extern "C" {
@@ -81,8 +85,8 @@ err_t cudaEventDestroy(void*) { return 0; }
 err_t cudaEventRecord(void* e, stream_t s) { op("record", s, e); return 0; }
 err_t cudaEventSynchronize(void*) { return 0; }
 err_t cudaEventElapsedTime(float* t, void*, void*) { *t = 1.f; return 0; }
-err_t cudaLaunchKernel(const void* f, dim3_, dim3_, void**, size_t, stream_t s) { return launch(f, s); }
-err_t cudaLaunchKernelExC(const config_t* c, const void* f, void**) { return launch(f, c->stream); }
+err_t cudaLaunchKernel(const void* f, dim3_, dim3_, void** args, size_t, stream_t s) { return launch(f, s, args); }
+err_t cudaLaunchKernelExC(const config_t* c, const void* f, void** args) { return launch(f, c->stream, args); }
 unsigned __cudaPushCallConfiguration(dim3_ g, dim3_ b, size_t m, stream_t s) { pushed = {g, b, m, s, 0, 0}; return 0; }
 err_t __cudaPopCallConfiguration(dim3_* g, dim3_* b, size_t* m, stream_t* s) {
     *g = pushed.grid; *b = pushed.block; *m = pushed.smem; *s = pushed.stream;
