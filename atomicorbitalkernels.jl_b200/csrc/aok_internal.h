@@ -289,6 +289,8 @@ int launch_ov3_f64(aok_plan* p, void* out, const void* posA, const void* posB, c
 // picks one of the two on the device
 namespace m3 {
 int setup_moments3(aok_plan* p);
+int reserve_moments3_f32(aok_plan* p, cudaError_t* e);
+int reserve_moments3_f64(aok_plan* p, cudaError_t* e);
 int launch_prepm3(aok_plan* p, int64_t B, cudaStream_t side);
 int launch_moments3_f32(aok_plan* p, void* out, const void* posA, const void* posB, const void* posC, int64_t B,
                         double lengthscale, cudaStream_t s);

@@ -327,10 +327,16 @@ int setup_moments3(aok_plan* p) {
     cudaError_t e = cudaMalloc(&sched, bytes);
     if (e == cudaSuccess) e = cudaMemcpy(sched, host.data(), host.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMalloc(&mom, (size_t)(tile * p->round3));
-    if (e != cudaSuccess) {
+    p->d_segsm = (int*)((char*)sched + at_segs);
+    int st = AOK_OK;
+    if (e == cudaSuccess)
+        st = p->prec == AOK_PREC_F64 ? reserve_moments3_f64(p, &e) : reserve_moments3_f32(p, &e);
+    if (e != cudaSuccess || st != AOK_OK) {
         if (sched) cudaFree(sched);
-        const int st = cuda_status(e, "3C overlap: moments");
-        p->no_mom3 = e == cudaErrorMemoryAllocation;
+        if (mom) cudaFree(mom);
+        p->d_segsm = nullptr;
+        if (st == AOK_OK) st = cuda_status(e, "3C overlap: moments");
+        p->no_mom3 = e == cudaErrorMemoryAllocation || e == cudaErrorLaunchOutOfResources;
         return p->no_mom3 ? AOK_OK : st;
     }
     char* base = (char*)sched;
@@ -340,7 +346,6 @@ int setup_moments3(aok_plan* p) {
     p->d_out3 = base + at_out;
     p->d_keym = (int*)(base + at_key);
     p->d_orderm = base + at_order;
-    p->d_segsm = (int*)(base + at_segs);
     p->d_cnt3 = (unsigned*)(base + at_cnt);
     p->d_mom3 = mom;
     return AOK_OK;

@@ -683,6 +683,24 @@ __global__ void __launch_bounds__(kTrThreads3, 1) k_transform3(const __grid_cons
     }
 }
 
+// Takes the local memory of the transform's routines from the device (1.6 GB of stack over
+// all SMs, which the driver keeps), through a launch that finds the tables picked and
+// returns: *e says whether there was room.
+template <typename FT>
+inline int reserve_moments3(aok_plan* p, cudaError_t* e) {
+    Ov3Params<FT> P;
+    memset(&P, 0, sizeof(P));
+    P.segs = p->d_segsm;
+    P.nitems = p->nitemsm;
+    auto tr = k_transform3<FT>;
+    const int st = kernel_prepare((const void*)tr, kTrSmem3, kTrThreads3, nullptr);
+    if (st != AOK_OK) return st;
+    *e = cudaMemsetAsync(p->d_segsm + p->nitemsm + 3, 0, sizeof(int), p->side);
+    if (*e == cudaSuccess) *e = launch_pdl(tr, dim3(p->num_sms), dim3(kTrThreads3), kTrSmem3, p->side, P);
+    if (*e == cudaSuccess) *e = cudaStreamSynchronize(p->side);
+    return AOK_OK;
+}
+
 template <typename FT>
 inline int launch_moments3(aok_plan* p, void* out, const void* posA, const void* posB, const void* posC, int64_t B,
                            double lengthscale, cudaStream_t s) {

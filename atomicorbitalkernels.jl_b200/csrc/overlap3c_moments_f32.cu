@@ -5,6 +5,8 @@
 namespace aok {
 namespace m3 {
 
+int reserve_moments3_f32(aok_plan* p, cudaError_t* e) { return reserve_moments3<float>(p, e); }
+
 int launch_moments3_f32(aok_plan* p, void* out, const void* posA, const void* posB, const void* posC, int64_t B,
                         double lengthscale, cudaStream_t s) {
     return launch_moments3<float>(p, out, posA, posB, posC, B, lengthscale, s);

@@ -27,6 +27,7 @@ static std::map<const void*, std::string> names;
 static std::string ops;
 static long nmalloc = 0, fail_at = -1, bad_frees = 0;
 static size_t fail_size = ~(size_t)0;
+static std::string fail_kernel;
 static err_t last = 0;
 static uintptr_t next_handle = 1;
 static config_t pushed;
@@ -41,12 +42,14 @@ static err_t launch(const void* f, stream_t s, void** args) {
     // the coefficient table that the kernel writes (first argument) or reads (fourth)
     const int coef = name.find("k_compile_coefI") != std::string::npos ? 0
                      : name.find("k_prep_pbI") != std::string::npos    ? 3 : -1;
+    if (!fail_kernel.empty() && name.find(fail_kernel) != std::string::npos) return note(OOM);
     op(("launch:" + name).c_str(), s, coef < 0 ? 0 : *(void**)args[coef]);
     return 0;
 }
 extern "C" {
 // the test's side
 void fake_fail(long at, size_t size) { nmalloc = 0; fail_at = at; fail_size = size; }
+void fake_fail_kernel(const char* name) { fail_kernel = name; }
 long fake_live() { return (long)live.size(); }
 long fake_bad_frees() { return bad_frees; }
 const char* fake_ops() { return ops.c_str(); }

@@ -1,5 +1,7 @@
 """Set-up of the 3-center overlap when device memory runs out, on a CUDA runtime without a
 device: a failed first call leaves nothing behind, and the next one starts again."""
+import pytest
+
 import fakecuda
 
 FIRST_CALL = """
@@ -50,7 +52,10 @@ for prec in (0, 1):
     for gb in (False, True):
         h = plan([0, 1, 2, 3], 3, 1 if gb else 2, prec, 5000)
         base = fake.fake_live()
-        fake.fake_fail(-1, 1 << 20)                # the moments want more than that
+        if WHAT == "buffer":
+            fake.fake_fail(-1, 1 << 20)            # the moments want more than that
+        else:
+            fake.fake_fail_kernel(b"k_transform3") # no local memory for its routines
         for repeat in range(2):
             ops()
             if gb:
@@ -65,8 +70,9 @@ print(json.dumps(dict(out=out, live=fake.fake_live(), bad=fake.fake_bad_frees())
 """
 
 
-def test_without_room_for_moments_the_tables_serve(tmp_path):
-    r = fakecuda.run(NO_ROOM, tmp_path)
+@pytest.mark.parametrize("what", ["buffer", "local memory"])
+def test_without_room_for_moments_the_tables_serve(tmp_path, what):
+    r = fakecuda.run(f"WHAT = {what!r}" + NO_ROOM, tmp_path)
     assert r["live"] == 0 and r["bad"] == 0
     assert len(r["out"]) == 8 and len({c["n"] for c in r["out"]}) == 1
     for c in r["out"]:
