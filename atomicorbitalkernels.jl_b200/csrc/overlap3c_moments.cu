@@ -14,13 +14,13 @@ namespace m3 {
 
 // Moments or explicit E tables (k_overlap3c).  The recursions on moments cost the same for
 // any number of primitive triples, the tables are rebuilt for each: moments are taken when a
-// function of a block sums at least two triples on average.  Measured (kernels, us, FP32C;
-// tables / moments for 1, 33 and 400 elements of two species): s shells of 3, 1, 1
-// primitives and p, d, f of one (mean 1.3) 67/116, 101/144, 148/219; s of 6, 3, 1 and p of
-// 3, 1 (mean 3.5) 143/117, 189/151, 273/227; two primitives in the f shell only (mean 2.7)
-// 364/131, 534/153, 642/235; two in every shell (mean 8) 424/135, 677/186, 1205/300.  FP64
-// the same (s of 3: 184/228 for 400, 6-3-1: 399/249).  The counts are on the device, so
-// both paths are launched and the one not taken returns at once.
+// function of a block sums at least two triples on average.  Measured (whole calls, us,
+// FP32C; tables / moments for 1, 33 and 400 elements of two species, 3 s, 2 p, d and f): s
+// shells of 3, 1, 1 primitives and the rest of one (mean 1.3) 74/118, 113/175, 155/213; s of
+// 6, 3, 1 and p of 3, 1 (mean 3.5) 155/124, 206/172, 268/215; two primitives in the f shell
+// only (mean 2.7) 359/129, 548/179, 654/221; two in every shell (mean 8) 392/130, 598/185,
+// 739/217.  FP64 the same (s of 3: 192/246 for 400, 6-3-1: 395/246).  The counts are on the
+// device, so both paths are launched and the one not taken returns at once.
 __device__ __forceinline__ void pick3(int* pick, const Item3* __restrict__ items, const int* pn, int n, int ns, int NZ) {
     __shared__ unsigned long long sums[2];
     if (threadIdx.x < 2) sums[threadIdx.x] = 0;
@@ -237,7 +237,9 @@ int setup_moments3(aok_plan* p) {
     const size_t fsz = p->prec == AOK_PREC_F64 ? sizeof(double) : sizeof(float);
     // Panels: per (B shell, C shell), runs of A shells whose blocks fit the CTA's slab; a
     // block too large for 32 elements is alone in its panel, which is taken once per group of
-    // elements.
+    // elements.  Panels of several blocks have as many elements in FP32 as in FP64, although
+    // the slab would take twice as many: fewer panels leave SMs idle (33 elements of 25
+    // functions, FP32: 235 -> 184 us; 777 of 32: 454 -> 428).
     const int room = fsz == 4 ? slab_room3<float>() : slab_room3<double>();
     auto fits = [&](int comps, int passes) { return ((comps + 1) | 1) * (32 / passes) <= room; };
     // the moment kernel's items: one per block, statically by class; slots of the moments
@@ -260,10 +262,8 @@ int setup_moments3(aok_plan* p) {
                 Panel3 pn{(short)sa, 0, (short)sb, (short)sc, 0, 1, 0, 0, 0, items[(size_t)(sc * ns + sb) * ns + sa].moff};
                 while (sa < ns && pn.nsa < kPanelItems3) {
                     const int la = (int)p->ls[sa], c = pn.comps + ncart(la) * ncart(lb) * ncart(lc);
-                    if (!fits(c, 1)) {
-                        if (pn.nsa) break;
-                        while (!fits(c, pn.passes)) pn.passes *= 2;
-                    }
+                    if (pn.nsa && ((c + 1) | 1) * 32 > slab_room3<double>()) break;
+                    while (!fits(c, pn.passes)) pn.passes *= 2;
                     pn.comps = c;
                     ++pn.nsa;
                     ++sa;
