@@ -19,8 +19,9 @@
 // primitive triple with explicit E tables.
 //
 // Prog3 lists these operations at compile time, depth first in the order of the
-// components (a value is formed right before its first use, to keep few alive);
-// NP > 1 splits the components by centre 0's component into NP programs.
+// components (a value is formed right before its first use, so that few are alive at a
+// time; in f-f-f, f-f-d and f-d-d still more than the registers hold).  NP > 1 splits the
+// components by centre 0's component into NP programs.
 #pragma once
 
 #include <utility>

@@ -136,9 +136,12 @@ struct DposParams {
 };
 
 // FP32: two CTAs of 8 warps per SM (<= 128 registers); FP64: one of 16 (4,000 pairs of 33
-// functions: 164 -> 121 us, of one of 8).  Bound by the latency of records and cotangent
-// rows: reading the records by 16-byte words took 8,191 pairs FP32 from 71 to 70 us, and
-// staging the cotangent panels through shared memory by cp.async lost (91 us).
+// functions: 121 us, with one of 8 164, although 128 registers instead of 255 put 992 bytes
+// a thread on the stack instead of 88).  Bound by the longest warp of a tile and by latency:
+// the warps wait at the tile's barrier (half of the cycles between issues in FP64, a
+// quarter in FP32) and for records and cotangent rows; the kernel issues in 11 % of the
+// cycles in FP64 and 19 % in FP32.  Staging the cotangent panels through shared memory by
+// cp.async lost (8,191 pairs FP32 70 -> 91 us).
 template <typename FT> constexpr int kDposWarps = sizeof(FT) == 4 ? 8 : 16;
 
 // exp(-mu R^2) of a record, mu, and its slot values by whole 16-byte words.

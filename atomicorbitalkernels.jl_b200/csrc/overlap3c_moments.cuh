@@ -24,12 +24,16 @@
 //
 // Bases with few primitives keep explicit E tables (pick3 in overlap3c_moments.cu).
 //
-// What bounds it: latency and instruction fetch.  The recursions are straight-line code run
-// once per (block, tile) by few warps, the moment sums a chain of exponentials.  777
-// elements of a 32-function basis of two elements (s to f, up to 8 primitives per shell):
-// 3,815 -> 472 us in FP64 (moments 210), 3,120 -> 444 us in FP32, against the routine with
-// explicit E tables per triple and run-time loops; 60 elements 2,280 -> 244 and 1,880 -> 225
-// us.  The output alone is 31 and 16 us.
+// What bounds it (777 elements of a 32-function basis of two elements, s to f, up to 8
+// primitives per shell; FP64, counters): k_moments3, 203 us, issues in 48 % of the cycles,
+// held up by the exponentials' arithmetic and by the barriers of shared blocks.
+// k_transform3, 262 us, issues in 13 % with 12 warps per SM: they wait at the barriers around
+// a panel's tasks, for moments and for values spilled to local memory (f-f-f parts spill 3
+// to 10 KB a thread, f-f-d up to 3, f-d-d up to 2.7, d-d-d 1), and for instructions, the
+// recursions being straight-line code run once per (block, tile).  Whole call, against the
+// routine with explicit E tables per triple and run-time loops: 3,815 -> 472 us in FP64,
+// 3,120 -> 428 in FP32; 60 elements 2,280 -> 244 and 1,880 -> 216.  The output alone is 31
+// and 16 us.
 // Tried: the recursions run by one warp per panel without barriers (2,600 us: one f block is
 // a long serial chain that holds up its whole panel); the moments summed in the same CTA as
 // a phase of their own (805 us).  Why the slab: stores straight from the lanes (each to its own
@@ -55,8 +59,8 @@ constexpr int kRecBytes3 = 3072;     // record buffer of a warp (k_moments3)
 constexpr int kMomSlots3 = 28;       // moments summed at a time (registers)
 // k_transform3 (<= 168 registers): one CTA of 12 warps per SM, whose slab holds the larger
 // blocks in fewer element groups than two CTAs of 6 warps would (777 elements of a
-// 32-function basis: FP64 500 against 577 us, FP32 484 against 527).  Shared memory:
-// geometry and slab.
+// 32-function basis: FP64 500 against 577 us, FP32 484 against 527 with FP64 exponentials).
+// Shared memory: geometry and slab.
 constexpr int kTrThreads3 = 384;
 constexpr int kTrSmem3 = 222 * 1024;
 
@@ -78,11 +82,12 @@ static_assert(class3(2, 2, 2) == 9 && class3(3, 0, 0) == 10 && class3(3, 3, 3) =
 // Moments and recursions are FP64 in both precisions.  With FP32 sums (runs of 8 triples
 // folded with TwoSum) and FP32 recursions up to d, p-p-p, d-p-p, d-d-p and d-d-d were off by up
 // to 1.3 times as much as with E tables (norm of the block, d-d-p of two primitives per shell:
-// 1.03e-7 against 8.2e-8); so they are off by 3e-8 to 4.7e-8 in every class, and 777 elements
-// take 444 us (FP32 sums and recursions: 488).  Up to d FP32 takes its exponentials from ex2
-// (rounding of the result apart, the error that is left); with FP64 ones every class is at
-// 2.5e-8 to 3.6e-8, but 777 elements take 484 us and 1,500 take 824 (758 with ex2).  Blocks
-// with an f shell have them in FP64, as their E tables do.
+// 1.03e-7 against 8.2e-8); so they are off by 3e-8 to 4.7e-8 in every class.  777 elements
+// take 428 us (490 so), 1,500 take 754 (757), 1,682 of a basis of up to 8 primitives in every
+// shell 976 (955).  Up to d FP32 takes its exponentials from ex2 (rounding of the result
+// apart, the error that is left); with FP64 ones every class is at 2.5e-8 to 3.6e-8, but 777
+// elements cost another 40 us and 1,500 another 65.  Blocks with an f shell have them in
+// FP64, as their E tables do.
 template <typename FT>
 __host__ __device__ constexpr bool fast_exp3(int l0) { return sizeof(FT) == 4 && l0 <= 2; }
 struct ClassInfo3 {
@@ -437,7 +442,7 @@ struct Ov3Params {
     const int4* tiles;
     const int* ntiles;
     unsigned* counter;   // [0] the moment kernel's, [1] the transform kernel's
-    const Item3* items;  // every block in queue order (k_prep3c)
+    const Item3* items;  // every block in queue order (k_prepm3)
     const int* segs;     // segment starts in items (nseg + 1 entries); nseg, H, pick at segs[nitems + 1], [nitems + 2], [nitems + 3]
     const Panel3* panels;
     const Out3* table;   // the panels' output elements
